@@ -191,7 +191,6 @@ struct StageIO<double> {
   static __device__ __forceinline__ const double* vg(const StageArgs& a) { return a.vg; }
   static __device__ __forceinline__ double* fs(const StageArgs& a) { return a.fs; }
   static __device__ __forceinline__ const double* fb(const StageArgs& a) { return a.fb; }
-  static __device__ __forceinline__ double* grad(const StageArgs& a) { return a.grad; }
   static __device__ __forceinline__ double* phi(const StageArgs& a) { return a.phi; }
 };
 template <>
@@ -200,7 +199,6 @@ struct StageIO<float> {
   static __device__ __forceinline__ const float* vg(const StageArgs& a) { return a.vg32; }
   static __device__ __forceinline__ float* fs(const StageArgs& a) { return a.fs32; }
   static __device__ __forceinline__ const float* fb(const StageArgs& a) { return a.fb32; }
-  static __device__ __forceinline__ float* grad(const StageArgs& a) { return a.grad32; }
   static __device__ __forceinline__ float* phi(const StageArgs& a) { return a.phi32; }
 };
 
@@ -533,15 +531,24 @@ struct DtFuse {
 //     a per-face bit turns S outward;
 //   * the vector from the centroid to the centroid of face m is
 //     (centroid - P_m) / 3.
-// gradient_node_kernel computes the same Green-Gauss gradient, min/max, Barth
-// limiter and reconstruction as the reference form, rearranged for fewer
-// instructions (agreement to round-off):
-//   grad V = 0.5/vol (sum_m V_m S_m + V_c sum_m S_m);
-//   phi = min(1, min_m A_m / D_m) with A_m = (V_max - V_c) or (V_c - V_min)
-//   and D_m = |grad V . r_m| + eps, the minimising face found by
-//   cross-multiplication, then one division per variable.
-// A missing face (a boundary face no marker lists) has S = r = 0 and points
-// at the cell itself, so it changes nothing.
+// The reconstruction of a tetrahedron needs no geometry. With lambda_m the
+// barycentric coordinate of vertex m, the outward normal of the face opposite it
+// is S_m = -3 vol grad(lambda_m), and r_m = (centroid - P_m) / 3, so for the
+// Green-Gauss gradient (Numerics.hpp:86-128) of the neighbours' values V_p
+//   grad V . r_m = -1/2 sum_p (V_p + V_c) grad(lambda_p) . (centroid - P_m)
+//                = -1/2 sum_p (V_p + V_c) (1/4 - [p = m]) = 1/2 (V_m - M),
+//   M = mean of the four neighbours' values.
+// gradient_node_kernel therefore reads only the cell's own and its neighbours'
+// primitives: no vertices, normals, volume or face codes (agreement with the
+// reference form to round-off). A missing face (a boundary face no marker
+// lists, FV_Grid.cpp:79-85) has S = r = 0 and names the cell itself; the sum
+// then runs over the listed faces, M = 1/4 sum_listed (V_p + V_c) - V_c.
+// The Barth limiter (Numerics.hpp:148-250) is
+//   phi = min(1, min_m A_m / D_m), A_m = (V_max - V_c) or (V_c - V_min) by the
+//   sign of grad V . r_m, D_m = |grad V . r_m| + eps;
+// A_m is the same for all faces of one sign, so only the largest and the
+// smallest increment count, and with the formula above those are the largest
+// and the smallest neighbour value. One division per variable.
 // ---------------------------------------------------------------------------
 // Ask the memory system to bring a line into L2 without holding a register;
 // the later load of the same address then waits on an L2 hit, not on DRAM.
@@ -602,25 +609,52 @@ __device__ __forceinline__ void face_normals(const T P[4][3], T S[4][3]) {
   face_normal<T, 3>(P, S[3]);
 }
 
+// Increments grad V . r_m of one variable from the neighbours' values minus
+// the cell's own, d_m, with limiter (barth): gr receives 1/2 (d_m - mean d),
+// and the limiter value is returned. n_missing faces are not listed (their d is
+// 0); shift is V_c (n_missing / 2), what they add to -M (0 for a closed cell).
+template <typename T>
+__device__ __forceinline__ T limited_increments(const T d[4], const int nb[4], int c, int n_missing, T shift, bool barth,
+                                                T gr[4]) {
+  const T mean = T(0.25) * ((d[0] + d[1]) + (d[2] + d[3])) - shift;
+#pragma unroll
+  for (int q = 0; q < 4; q++) gr[q] = T(0.5) * (d[q] - mean);
+  if (!barth) return T(1);
+  // extremes of two pairs, one comparison each
+  const bool s01 = d[0] < d[1], s23 = d[2] < d[3];
+  const T l0 = s01 ? d[0] : d[1], h0 = s01 ? d[1] : d[0], l1 = s23 ? d[2] : d[3], h1 = s23 ? d[3] : d[2];
+  const T dmax = rmax(h0, h1), dmin = rmin(l0, l1);
+  T ghi = T(0.5) * (dmax - mean), glo = T(0.5) * (dmin - mean);
+  if (n_missing) {  // listed faces only
+    ghi = glo = T(0);
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+      if (nb[q] != c) {
+        ghi = rmax(ghi, gr[q]);
+        glo = rmin(glo, gr[q]);
+      }
+  }
+  T An = T(1), Dn = T(1);  // best ratio so far, starting at 1
+  const T Ah = rmax(dmax, T(0)), Dh = ghi + Gas<T>::eps;   // V_max - V_c
+  const T Al = rmax(-dmin, T(0)), Dl = Gas<T>::eps - glo;  // V_c - V_min
+  if (ghi > T(0) && Ah < Dh) {
+    An = Ah;
+    Dn = Dh;
+  }
+  const bool better = glo < T(0) && Al * Dn < An * Dl;
+  An = better ? Al : An;
+  Dn = better ? Dl : Dn;
+  return An * nr_rcp(Dn);
+}
+
 // kPipe: 0 one variable's loads at a time; 1 the next variable's loads in
 // flight during this one's arithmetic; 2 all five variables' loads issued
 // together before any arithmetic (one exposed memory latency instead of five,
 // at the cost of registers); 3 as 0, with the cell's own rows prefetched
 // into L2 first.
 // The body for one cell; vown receives the cell's own primitives.
-// CFL time step of one cell from its primitives with the fast forms'
-// reciprocal and reciprocal square root (within 2 ulp of dt_of_cell).
-__device__ __forceinline__ double dt_of_cell_fast(const double V[5], double dS0, double dS1, double dS2, double vol,
-                                                  double cfl) {
-  const double g = Gas<double>::gamma * V[4];
-  const double cs = g * nr_rsqrt(g * V[0]);  // sqrt(gamma p / rho)
-  const double sum = fma(fabs(V[3]) + cs, dS2, fma(fabs(V[2]) + cs, dS1, (fabs(V[1]) + cs) * dS0));
-  return cfl * vol * nr_rcp(sum);
-}
-
-template <typename T, int kPipe, bool kDS = false>
-__device__ __forceinline__ void gradient_node_cell(const MeshView<T>& m, const StageArgs& a, int c, T vown[5],
-                                                   T* dS_out = nullptr) {
+template <typename T, int kPipe>
+__device__ __forceinline__ void gradient_node_cell(const MeshView<T>& m, const StageArgs& a, int c, T vown[5]) {
   const int st = m.stride;
   const T* __restrict__ Vin = StageIO<T>::vin(a);
   const T* __restrict__ Vg = StageIO<T>::vg(a);
@@ -650,92 +684,25 @@ __device__ __forceinline__ void gradient_node_cell(const MeshView<T>& m, const S
   [[maybe_unused]] T vcN, voN[4];
   [[maybe_unused]] T vcA[5], voA[5][4];
   if constexpr (kPipe == 2) {
-    // the same loads as fetch(), all five variables' at once
 #pragma unroll
-    for (int k = 0; k < 5; k++) vcA[k] = Vin[size_t(k) * st + c];
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const bool cell = nb[q] >= 0;
-      const auto* p = cell ? Vin + nb[q] : Vg + (-nb[q] - 1);
-      const size_t rs = cell ? size_t(st) : size_t(m.bstride);
-#pragma unroll
-      for (int k = 0; k < 5; k++) voA[k][q] = p[k * rs];
-    }
+    for (int k = 0; k < 5; k++) fetch(k, vcA[k], voA[k]);
   } else if (kPipe == 1) {
     fetch(0, vcN, voN);
   }
-  const int code = m.gcode[c];
-  T S[4][3], d[4][3];  // outward normals; (centroid - P_m) / 3
-  {
-    T P[4][3];
-    load_vertices(m, c, P, a.status);
-    face_normals(P, S);
-    const T cen[3] = {T(0.25) * ((P[0][0] + P[1][0]) + (P[2][0] + P[3][0])),
-                      T(0.25) * ((P[0][1] + P[1][1]) + (P[2][1] + P[3][1])),
-                      T(0.25) * ((P[0][2] + P[1][2]) + (P[2][2] + P[3][2]))};
+  int n_missing = 0;
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const int bits = code >> (3 * q);
-      const T sgn = (bits & 1) == 0 ? T(0) : ((bits & 2) ? T(-1) : T(1));  // 0: no face
-#pragma unroll
-      for (int e = 0; e < 3; e++) {
-        S[q][e] *= sgn;
-        d[q][e] = (bits & 1) ? (cen[e] - P[q][e]) * T(1.0 / 3.0) : T(0);
-      }
-    }
-  }
-  const T ssum[3] = {(S[0][0] + S[1][0]) + (S[2][0] + S[3][0]), (S[0][1] + S[1][1]) + (S[2][1] + S[3][1]),
-                     (S[0][2] + S[1][2]) + (S[2][2] + S[3][2])};
-  if constexpr (kDS) {
-    // projected areas of calc_Delta_S (Solver.cpp:276-298): half the sum of
-    // |S_d| over the cell's interior faces, from the normals in registers
-#pragma unroll
-    for (int e = 0; e < 3; e++) {
-      T acc = T(0);
-#pragma unroll
-      for (int q = 0; q < 4; q++) acc += nb[q] >= 0 ? fabs(S[q][e]) : T(0);
-      dS_out[e] = T(0.5) * acc;
-    }
-  }
-  const T hv = T(0.5) * nr_rcp(T(m.vol[c]));
+  for (int q = 0; q < 4; q++) n_missing += nb[q] == c;
   const bool rat = a.barth && ratchet_on(a, c);
   auto variable = [&](int k, T vc, const T vo[4]) {
     vown[k] = vc;
-    T acc[3];
+    T d[4], gr[4];
 #pragma unroll
-    for (int e = 0; e < 3; e++) {
-      acc[e] = vc * ssum[e];
-#pragma unroll
-      for (int q = 0; q < 4; q++) acc[e] = fma(vo[q], S[q][e], acc[e]);
-    }
-    const T g[3] = {hv * acc[0], hv * acc[1], hv * acc[2]};
-    const T vmax = fmax(fmax(fmax(vc, vo[0]), fmax(vo[1], vo[2])), vo[3]);
-    const T vmin = fmin(fmin(fmin(vc, vo[0]), fmin(vo[1], vo[2])), vo[3]);
-    T gr[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) gr[q] = fma(g[2], d[q][2], fma(g[1], d[q][1], g[0] * d[q][0]));
-    T phi = T(1);
-    if (a.barth) {
-      T An = T(1), Dn = T(1);  // best ratio so far, starting at 1
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const T d2 = gr[q];
-        const T A = d2 > T(0) ? vmax - vc : vc - vmin;
-        const T D = fabs(d2) + Gas<T>::eps;
-        const bool better = (d2 != T(0)) && (A * Dn < An * D);
-        An = better ? A : An;
-        Dn = better ? D : Dn;
-      }
-      phi = An * nr_rcp(Dn);
-      if (rat) phi = ratchet(a, size_t(k) * st + c, phi);
-    }
+    for (int q = 0; q < 4; q++) d[q] = vo[q] - vc;
+    T phi = limited_increments(d, nb, c, n_missing, T(0.5) * T(n_missing) * vc, a.barth != 0, gr);
+    if (rat) phi = ratchet(a, size_t(k) * st + c, phi);
 #pragma unroll
     for (int q = 0; q < 4; q++) fsc[size_t(q * 5 + k) * st] = fma(phi, gr[q], vc);
-    if (T* gdump = StageIO<T>::grad(a)) {
-#pragma unroll
-      for (int e = 0; e < 3; e++) gdump[(k * 3 + e) * st + c] = g[e];
-      StageIO<T>::phi(a)[k * st + c] = phi;
-    }
+    if (T* pdump = StageIO<T>::phi(a)) pdump[k * st + c] = phi;
   };
   if constexpr (kPipe == 2) {
 #pragma unroll
@@ -757,6 +724,15 @@ __device__ __forceinline__ void gradient_node_cell(const MeshView<T>& m, const S
   }
 }
 
+// CFL time step of one cell from its primitives with the fast forms'
+// reciprocal and reciprocal square root (within 2 ulp of dt_of_cell).
+__device__ __forceinline__ double dt_of_cell_fast(const double V[5], double dS0, double dS1, double dS2, double vol,
+                                                  double cfl) {
+  const double g = Gas<double>::gamma * V[4];
+  const double cs = g * nr_rsqrt(g * V[0]);  // sqrt(gamma p / rho)
+  const double sum = fma(fabs(V[3]) + cs, dS2, fma(fabs(V[2]) + cs, dS1, (fabs(V[1]) + cs) * dS0));
+  return cfl * vol * nr_rcp(sum);
+}
 
 // kDt: also the next step's time step from the cell's own primitives, after
 // the gradient work (the FP64 form's last stage; the primitives are those of
@@ -770,21 +746,62 @@ __global__ void __launch_bounds__(128, kMinBlocks) gradient_node_kernel(MeshView
   pdl_wait_previous();
   const bool in = c < m.n;
   const bool active = in && !frozen_cell(a, c);
-  T vown[5], dS[3];
-  if (active) gradient_node_cell<T, kPipe, kDt>(m, a, c, vown, dS);
+  T vown[5];
+  if (active) gradient_node_cell<T, kPipe>(m, a, c, vown);
   if constexpr (kDt) {
     double dtc = DBL_MAX;
     if (in) {
       if (!active) {
         if (dtf.dt_next) dtf.dt_next[c] = 0.0;  // a converged case keeps its state
       } else {
-        const double d = dt_of_cell_fast(vown, dS[0], dS[1], dS[2], m.vol[c], dtf.cfl);
+        const double d =
+            dt_of_cell_fast(vown, m.dS[c], m.dS[m.stride + c], m.dS[2 * m.stride + c], m.vol[c], dtf.cfl);
         if (dtf.dt_next) dtf.dt_next[c] = d;
         if (!(d > 0.0) && !isnan(d)) atomicOr(a.status, kErrDt);
         if (d > 0.0) dtc = d;  // std::min skips NaN (comparisons with NaN are false)
       }
     }
     warp_min_to(dtc, dtf.dt_min_bits);
+  }
+}
+
+// The Green-Gauss gradient itself (calc_green_gauss_gradient, Numerics.hpp:86-128)
+// for nf_get_field: the step never reads it, so it is computed apart, only
+// where the stage fields are kept. One thread per cell, from the primitives V
+// and ghosts Vg in FP64 or FP32, into out [15][stride] (k*3+d).
+template <typename T, typename Vt>
+__global__ void __launch_bounds__(128) gradient_field_kernel(MeshView<T> m, StageArgs a, const Vt* __restrict__ V,
+                                                             const Vt* __restrict__ Vg, T* __restrict__ out) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= m.n || frozen_cell(a, c)) return;
+  const int st = m.stride;
+  const int code = m.gcode[c];
+  T P[4][3], S[4][3], ssum[3] = {T(0), T(0), T(0)};
+  load_vertices(m, c, P, a.status);
+  face_normals(P, S);
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const int bits = code >> (3 * q);
+    const T sgn = (bits & 1) == 0 ? T(0) : ((bits & 2) ? T(-1) : T(1));  // 0: no face
+#pragma unroll
+    for (int e = 0; e < 3; e++) ssum[e] += (S[q][e] *= sgn);
+  }
+  const bool closed = (code & 0x249) == 0x249;  // the listed normals sum to zero
+  const double ivol = 1.0 / m.vol[c];
+  for (int k = 0; k < 5; k++) {
+    const Vt vc = V[size_t(k) * st + c];
+    T g[3] = {T(0), T(0), T(0)};
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int nb = checked_nb(m.nbvf[q * st + c], 0, m.n, m.nb, c, a.status);
+      const T d = T((nb >= 0 ? V[size_t(k) * st + nb] : Vg[size_t(k) * m.bstride + (-nb - 1)]) - vc);
+#pragma unroll
+      for (int e = 0; e < 3; e++) g[e] = fma(d, S[q][e], g[e]);
+    }
+#pragma unroll
+    for (int e = 0; e < 3; e++)
+      out[size_t(k * 3 + e) * st + c] =
+          T(0.5 * ivol) * g[e] + (closed ? T(0) : T(double(vc) * double(ssum[e]) * ivol));
   }
 }
 

@@ -101,6 +101,7 @@ void launch_gradient_fast(const MeshView<double>& m, const StageArgs& a, const D
   const DtFuse d = dt ? *dt : DtFuse{0.0, nullptr, nullptr};
   if (dt) NF_GRAD_DISPATCH(true);
   else NF_GRAD_DISPATCH(false);
+  if (a.grad) gradient_field_kernel<double, double><<<grid_for(m.n, 128), 128, 0, l.stream>>>(m, a, a.Vin, a.vg, a.grad);
 }
 #undef NF_GRAD_DISPATCH
 void launch_flux_fast(const MeshView<double>& m, const StageArgs& a, Launch l) {
@@ -127,6 +128,7 @@ void launch_flux_fast(const MeshView<double>& m, const StageArgs& a, Launch l) {
 
 void launch_gradient_mixed(const MeshView<float>& m, const StageArgs& a, Launch l) {
   NF_DELTA_DISPATCH(gradient_delta_kernel, m, a, l);
+  if (a.grad32) gradient_field_kernel<float, double><<<grid_for(m.n, 128), 128, 0, l.stream>>>(m, a, a.Vin, a.vg, a.grad32);
 }
 void launch_flux_mixed(const MeshView<float>& m, const StageArgs& a, Launch l) {
   NF_DELTA_DISPATCH(flux_delta_kernel, m, a, l);
@@ -186,6 +188,7 @@ void launch_gradient_m32(const MeshView<float>& m, const StageArgs& a, Launch l)
     case 9: launch_pdl(gradient_node_kernel<float, 3, kCap2<float>, false>, g, b, l.stream, m, a, d); break;
     default: launch_pdl(gradient_node_kernel<float, 0, 1, false>, g, b, l.stream, m, a, d); break;
   }
+  if (a.grad32) gradient_field_kernel<float, float><<<g, b, 0, l.stream>>>(m, a, a.Vin32, a.vg32, a.grad32);
 }
 void launch_flux_m32(const MeshView<float>& m, const StageArgs& a, Launch l) {
   NF_NODE_DISPATCH(flux_node_kernel, float, m, a, l);

@@ -69,9 +69,11 @@ __device__ __forceinline__ void rusanov_delta(const float vc[5], const float dL[
   for (int k = 0; k < 5; k++) F[k] = h * fmaf(-smax, R.dU[k] - L.dU[k], L.dF[k] + R.dF[k]);
 }
 
-// Gradient, min/max, Barth limiter (FLT_EPSILON, as the reference's
-// single-precision build, Numerics.hpp:171) and the reconstruction increments
-// phi grad V . r_m, one thread per cell, from FP64 primitives and ghosts.
+// Limiter (FLT_EPSILON, as the reference's single-precision build,
+// Numerics.hpp:171) and the reconstruction increments phi grad V . r_m, one
+// thread per cell, from the differences of FP64 primitives and ghosts: like
+// gradient_node_kernel it needs no geometry (kernels.cuh), so the increments
+// carry no rounding of FP32 vertices either.
 template <int kPipe, int kMinBlocks>
 __global__ void __launch_bounds__(128, kMinBlocks) gradient_delta_kernel(MeshView<float> m, StageArgs a) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -85,11 +87,19 @@ __global__ void __launch_bounds__(128, kMinBlocks) gradient_delta_kernel(MeshVie
   int nb[4];
 #pragma unroll
   for (int q = 0; q < 4; q++) nb[q] = checked_nb(m.nbvf[q * st + c], 0, m.n, m.nb, c, a.status);
-  auto fetch = [&](int k, double& vc, double vo[4]) {
-    const double* Vk = V + size_t(k) * st;
-    vc = Vk[c];
+  // each face's row base and row stride (a cell's or a ghost's) chosen once
+  const double* qb[4];
+  int qs[4];
 #pragma unroll
-    for (int q = 0; q < 4; q++) vo[q] = nb[q] >= 0 ? Vk[nb[q]] : Vg[k * m.bstride + (-nb[q] - 1)];
+  for (int q = 0; q < 4; q++) {
+    const bool cell = nb[q] >= 0;
+    qb[q] = cell ? V + nb[q] : Vg + (-nb[q] - 1);
+    qs[q] = cell ? st : m.bstride;
+  }
+  auto fetch = [&](int k, double& vc, double vo[4]) {
+    vc = V[size_t(k) * st + c];
+#pragma unroll
+    for (int q = 0; q < 4; q++) vo[q] = qb[q][k * qs[q]];
   };
   if constexpr (kPipe == 3) {
 #pragma unroll
@@ -98,89 +108,24 @@ __global__ void __launch_bounds__(128, kMinBlocks) gradient_delta_kernel(MeshVie
   [[maybe_unused]] double vcN, voN[4];
   [[maybe_unused]] double vcA[5], voA[5][4];
   if constexpr (kPipe == 2) {
-    // the same loads as fetch(), with each face's row base and row stride
-    // chosen once (cell row or ghost row) instead of per variable
 #pragma unroll
-    for (int k = 0; k < 5; k++) vcA[k] = V[size_t(k) * st + c];
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const bool cell = nb[q] >= 0;
-      const auto* p = cell ? V + nb[q] : Vg + (-nb[q] - 1);
-      const size_t rs = cell ? size_t(st) : size_t(m.bstride);
-#pragma unroll
-      for (int k = 0; k < 5; k++) voA[k][q] = p[k * rs];
-    }
+    for (int k = 0; k < 5; k++) fetch(k, vcA[k], voA[k]);
   } else if (kPipe == 1) {
     fetch(0, vcN, voN);
   }
-  const int code = m.gcode[c];
-  float S[4][3], d[4][3];  // outward normals; (centroid - P_m) / 3
-  {
-    float P[4][3];
-    load_vertices(m, c, P, a.status);
-    face_normals(P, S);
-    const float cen[3] = {0.25f * ((P[0][0] + P[1][0]) + (P[2][0] + P[3][0])),
-                          0.25f * ((P[0][1] + P[1][1]) + (P[2][1] + P[3][1])),
-                          0.25f * ((P[0][2] + P[1][2]) + (P[2][2] + P[3][2]))};
+  int n_missing = 0;
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const int bits = code >> (3 * q);
-      const float sgn = (bits & 1) == 0 ? 0.f : ((bits & 2) ? -1.f : 1.f);  // 0: no face
-#pragma unroll
-      for (int e = 0; e < 3; e++) {
-        S[q][e] *= sgn;
-        d[q][e] = (bits & 1) ? (cen[e] - P[q][e]) * (1.0f / 3.0f) : 0.f;
-      }
-    }
-  }
-  const float hv = float(0.5 / m.vol[c]);
+  for (int q = 0; q < 4; q++) n_missing += nb[q] == c;
   const bool rat = a.barth && ratchet_on(a, c);
   auto variable = [&](int k, double vc, const double vo[4]) {
-    float dv[4];
+    float d[4], gr[4];
 #pragma unroll
-    for (int q = 0; q < 4; q++) dv[q] = float(vo[q] - vc);
-    float acc[3];
-#pragma unroll
-    for (int e = 0; e < 3; e++) {
-      acc[e] = dv[0] * S[0][e];
-#pragma unroll
-      for (int q = 1; q < 4; q++) acc[e] = fmaf(dv[q], S[q][e], acc[e]);
-    }
-    float g[3] = {hv * acc[0], hv * acc[1], hv * acc[2]};
-    if ((code & 0x249) != 0x249) {
-      // a dropped boundary face (FV_Grid.cpp:79-85): the listed normals do not
-      // sum to zero, grad = grad_diff + V_c sum_listed S / vol
-#pragma unroll
-      for (int e = 0; e < 3; e++)
-        g[e] += float(vc * double((S[0][e] + S[1][e]) + (S[2][e] + S[3][e])) / m.vol[c]);
-    }
-    const float up = fmaxf(fmaxf(fmaxf(0.f, dv[0]), fmaxf(dv[1], dv[2])), dv[3]);   // V_max - V_c
-    const float dn = fminf(fminf(fminf(0.f, dv[0]), fminf(dv[1], dv[2])), dv[3]);   // V_min - V_c
-    float gr[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) gr[q] = fmaf(g[2], d[q][2], fmaf(g[1], d[q][1], g[0] * d[q][0]));
-    float phi = 1.f;
-    if (a.barth) {
-      float An = 1.f, Dn = 1.f;
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const float d2 = gr[q];
-        const float A = d2 > 0.f ? up : -dn;
-        const float D = fabsf(d2) + Gas<float>::eps;
-        const bool better = (d2 != 0.f) && (A * Dn < An * D);
-        An = better ? A : An;
-        Dn = better ? D : Dn;
-      }
-      phi = An * nr_rcp(Dn);
-      if (rat) phi = ratchet(a, size_t(k) * st + c, phi);
-    }
+    for (int q = 0; q < 4; q++) d[q] = float(vo[q] - vc);
+    float phi = limited_increments(d, nb, c, n_missing, float(0.5 * n_missing * vc), a.barth != 0, gr);
+    if (rat) phi = ratchet(a, size_t(k) * st + c, phi);
 #pragma unroll
     for (int q = 0; q < 4; q++) inc_c[size_t(q * 5 + k) * st] = phi * gr[q];
-    if (a.grad32) {
-#pragma unroll
-      for (int e = 0; e < 3; e++) a.grad32[(k * 3 + e) * st + c] = g[e];
-      a.phi32[k * st + c] = phi;
-    }
+    if (a.phi32) a.phi32[k * st + c] = phi;
   };
   if constexpr (kPipe == 2) {
 #pragma unroll
