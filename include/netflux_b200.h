@@ -177,7 +177,7 @@ typedef struct {
   int n_patches;
   double freestream[5]; /* Config::get_primvars_inf (rho,u,v,w,p) */
   int block_size;       /* 0: library default; > 0: fixed block size of the
-                           gradient and flux kernels (no tuning) */
+                           kernels that have a choice (no tuning) */
   int kernel_variant;   /* with block_size > 0: fast-kernel variant (see nf_tune) */
   /* Limiter ratchet (extension; the reference's Barth limiter is always live,
    * Numerics.hpp:148-250, and its residual stalls near a 1e-3 drop on steady
@@ -329,27 +329,27 @@ int nf_get_field(nf_solver* s, int which, double* out, int64_t n_values);
 /* Wait for queued work; report a device-side validity failure. */
 int nf_synchronize(nf_solver* s);
 
-/* Time the launch shapes of the gradient and flux kernels on the current
- * state and keep the fastest: block size (64 or 128 threads), whether each
- * thread issues its next variable's / face's loads before the current
- * arithmetic (variants 1, 3, 5), all of its loads before any arithmetic
- * (variants 6, 7), or L2 prefetches of its own rows first (variants 8, 9),
- * and a register cap for occupancy (none, variants 0-1 and 6; 6 / 8 resident
- * 128-thread blocks for FP64 / FP32, variants 2-3 and 8; 7 / 9, variants 4-5
- * and 9; 4 / 5, variant 7). config (may be NULL) receives {gradient block, gradient
- * variant, flux block, flux variant}. The state is unchanged. The reference
- * has no counterpart (it runs on one CPU thread). */
+/* The form with FP32 copies under the Barth limiter: time the launch shapes of
+ * its gradient and flux kernels on the current state and keep the fastest: block
+ * size (64 or 128 threads), how loads are issued (variants 1, 3, 5 software
+ * pipelined, 6 and 7 all before any arithmetic, 8 and 9 after L2 prefetches of
+ * the cell's own rows) and a register cap for occupancy (none, variants 0-1 and
+ * 6; 8 resident 128-thread blocks, variants 2-3 and 8; 9, variants 4-5 and 9; 5,
+ * variant 7). The other forms' stage kernel has one shape, which follows from the
+ * mesh, so for them nothing is timed. config (may be NULL) receives {gradient
+ * block, gradient variant, flux block, flux variant}. The state is unchanged. The
+ * reference has no counterpart (it runs on one CPU thread). */
 int nf_tune(nf_solver* s, int* config);
 /* Fix the launch shapes instead of timing them: config = {gradient block,
  * gradient variant, flux block, flux variant} as nf_tune reports them (block
- * 32..128 in steps of 32, variant 0..9); NF_ERR_ARG otherwise. Used to
- * profile a given shape. No counterpart in the reference. */
+ * 32..128 in steps of 32, variant 0..9); NF_ERR_ARG otherwise. Accepted for every
+ * form. Used to profile a given shape. No counterpart in the reference. */
 int nf_set_launch_shapes(nf_solver* s, const int* config);
 
 /* Kernel classes reported by nf_time_steps. */
 #define NF_KERNEL_TIMESTEP 0
-#define NF_KERNEL_GRADIENT 1
-#define NF_KERNEL_FLUX 2
+#define NF_KERNEL_GRADIENT 1   /* where it is a kernel of its own, and kept gradient fields */
+#define NF_KERNEL_FLUX 2       /* or the stage kernel */
 #define NF_KERNEL_OTHER 3
 #define NF_KERNEL_COUNT 4
 

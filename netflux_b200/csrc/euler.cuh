@@ -53,31 +53,38 @@ struct PatchBC {
 };
 
 // Reciprocal and reciprocal square root for the fast forms, by the
-// Newton-Raphson method from a single-precision hardware estimate: each
-// iteration roughly doubles the number of correct bits (about 2^-22 after the
-// estimate, 2^-44 after one step, beyond double precision after two), so the
-// FP64 results are within about 1 ulp; FP32 uses the hardware estimate
-// directly (within about 1 ulp of the correctly rounded value). The FP64
-// forms start from the correctly rounded FP32 reciprocal: with the bare
-// estimate there the FP64 gradient kernel measured 17 % slower at 3.1M tets.
-// Operands are positive, normal and within single-precision range (densities,
-// pressures, |S|^2, volumes).
-// the hardware's single-precision reciprocal estimate (PTX rcp.approx.ftz.f32,
-// relative error below 2^-23 for the normal operands used here)
+// Newton-Raphson method from a hardware estimate: each iteration roughly doubles
+// the number of correct bits, so the FP64 results, two iterations from an
+// estimate of about 20 bits, are within about 1 ulp; FP32 uses the hardware
+// estimate directly (within about 1 ulp of the correctly rounded value). The
+// FP64 estimates are the FP64-range ones (PTX rcp.approx.ftz.f64,
+// rsqrt.approx.ftz.f64), which need no conversion to FP32 and back: with FP32
+// estimates a stage of 3.1M tets took 396 us, with these 369 us.
+// Operands are positive and normal (densities, pressures, |S|^2, volumes).
 __device__ __forceinline__ float rcp_estimate(float x) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
+__device__ __forceinline__ double rcp_estimate(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  return r;
+}
+__device__ __forceinline__ double rsqrt_estimate(double x) {
+  double r;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  return r;
+}
 __device__ __forceinline__ double nr_rcp(double b) {
-  double r = double(__frcp_rn(float(b)));
+  double r = rcp_estimate(b);
   double e = fma(-b, r, 1.0);
   r = fma(r, e, r);
   e = fma(-b, r, 1.0);
   return fma(r, e, r);
 }
 __device__ __forceinline__ double nr_rsqrt(double x) {
-  double r = double(rsqrtf(float(x)));
+  double r = rsqrt_estimate(x);
   const double h = 0.5 * x;
   double e = fma(-h * r, r, 0.5);  // r <- r (3/2 - x r^2 / 2)
   r = fma(r, e, r);
@@ -184,7 +191,12 @@ __device__ __forceinline__ void rusanov_fast(const T VL[5], const T VR[5], const
 
 // ---- boundary conditions (Numerics.cpp:59-171) on primitive states ----
 // n is S.normalized() of the face (S points out of the domain).
-template <typename T>
+// kRef: the far field's two powers by pow(), as the reference. Else without: with
+// gamma = 7/5 the ghost density (gamma s_b / c_b^2)^(1/(gamma-1)) of an outflow,
+// s_b = p rho^-gamma, is y^(5/2) / rho^(7/2), y = gamma p / c_b^2, and of an
+// inflow y^(5/2) with y = gamma s_b / c_b^2, half powers being square roots. The
+// exponents differ from the reference's rounded ones by 4e-16.
+template <typename T, bool kRef = true>
 __device__ __forceinline__ void ghost_state(const PatchBC& bc, const T V[5], const T n[3], T G[5]) {
   if (bc.type == kBcSlip) {  // BC_SlipWall
     const T vn = (V[1] * n[0] + V[2] * n[1]) + V[3] * n[2];
@@ -204,22 +216,23 @@ __device__ __forceinline__ void ghost_state(const PatchBC& bc, const T V[5], con
     const T Rm = (vn_fs - c_fs > T(0)) ? vn_d - T(2) * c_d / g1 : vn_fs - T(2) * c_fs / g1;
     const T vn_b = T(0.5) * (Rp + Rm);
     const T c_b = g1 / T(4) * (Rp - Rm);
-    T s_b;
-    if (vn_fs > T(0)) {
-      G[1] = V[1] + (vn_b - vn_d) * n[0];
-      G[2] = V[2] + (vn_b - vn_d) * n[1];
-      G[3] = V[3] + (vn_b - vn_d) * n[2];
-      s_b = V[4] * pow(V[0], -gam);
-    } else {
-      G[1] = vfs[0] + (vn_fs - vn_b) * n[0];
-      G[2] = vfs[1] + (vn_fs - vn_b) * n[1];
-      G[3] = vfs[2] + (vn_fs - vn_b) * n[2];
-      s_b = T(bc.s_fs);
-    }
+    const bool outflow = vn_fs > T(0);
+#pragma unroll
+    for (int d = 0; d < 3; d++)
+      G[1 + d] = outflow ? V[1 + d] + (vn_b - vn_d) * n[d] : vfs[d] + (vn_fs - vn_b) * n[d];
     // Numerics.cpp:149 computes (gamma s / c^2)^(1/(gamma-1)), the inverse of
     // the isentropic density; it is exact only for rho = 1 (kept by default)
-    const T rho_b = bc.density_fix ? pow(c_b * c_b / (gam * s_b), Gas<T>::g1_inv)
-                                   : pow(gam * s_b / (c_b * c_b), Gas<T>::g1_inv);
+    T rho_b;
+    if constexpr (kRef) {
+      const T s_b = outflow ? V[4] * pow(V[0], -gam) : T(bc.s_fs);
+      rho_b = bc.density_fix ? pow(c_b * c_b / (gam * s_b), Gas<T>::g1_inv)
+                             : pow(gam * s_b / (c_b * c_b), Gas<T>::g1_inv);
+    } else {
+      const T y = gam * (outflow ? V[4] : T(bc.s_fs)) / (c_b * c_b);
+      const T up = y * y * sqrt(y);
+      const T down = outflow ? V[0] * V[0] * V[0] * sqrt(V[0]) : T(1);
+      rho_b = bc.density_fix ? down / up : up / down;
+    }
     G[0] = rho_b;
     G[4] = c_b * c_b * rho_b / gam;
   } else {  // BC_NoSlipWall

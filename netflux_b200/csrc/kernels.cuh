@@ -1,4 +1,6 @@
-// Per-cell gather kernels of one explicit step on the device mesh.
+// Per-cell gather kernels of one explicit step on the device mesh: the
+// reference-order form whole, and what the fast forms' stage kernel
+// (kernels_tile.cuh) is made of.
 //
 // Layout (all arrays resident in HBM for the whole run; cell c is the c-th
 // cell along the Hilbert curve):
@@ -22,10 +24,11 @@
 //               centroid of each of its faces (r_i or r_j of the face)
 //   boundary    b_cell, b_slot, b_face, b_patch : [nb]; ghost states vg and
 //               boundary fluxes fb : [5][bstride]
-// Each face's flux is evaluated by both of its cells with the owner on the
-// left, so both see bit-identical values; no atomics, deterministic results.
-// The gradient kernel runs one thread per (cell, variable), the flux kernel
-// four threads per cell (one per face slot).
+// The slots, face states, face arrays and boundary fluxes are the
+// reference-order form's. Each face's flux is evaluated by both of its cells, so
+// that both see bit-identical values; no atomics, deterministic results. The
+// reference-order gradient kernel runs one thread per (cell, variable), its flux
+// kernel four threads per cell (one per face slot).
 #pragma once
 
 #include <type_traits>
@@ -65,7 +68,6 @@ struct MeshView {
   const int* __restrict__ b_slot;  // owner's slot of the face
   const int* __restrict__ b_face;  // face id (geometry)
   const int* __restrict__ b_patch; // patch
-  const int* __restrict__ b_fs;    // face-state slot of the owner (slot order of the kernels in use)
   int n_nodes;                     // for the index checks of NF_DEBUG builds
   int n_patches;
 };
@@ -116,27 +118,34 @@ struct StageArgs {
   const double* dt_local;
   const double* scal;    // device scalars: [0] dt (min target), [1] time, [2] t_end
   unsigned* status;
-  // mixed form: FP32 reconstruction increments and fields
+  // mixed forms: kept stage fields; FP32 copies under the limiter: face states
+  // [4][5][stride] and boundary fluxes [5][bstride]
   float* fs32;
+  float* fb32;
   float* grad32;
   float* phi32;
   // boundary faces: cell-centre ghost states [5][bstride] and boundary fluxes
-  // [5][bstride] (mixed form: FP32 differences to the owner's physical flux)
+  // [5][bstride] (reference-order form)
   double* vg;
   double* fb;
-  float* fb32;
   // mixed form with FP32 copies (NF_PREC_MIXED32): the FP32 primitives of
-  // the stage input and of its result, and FP32 ghost states [5][bstride];
-  // the face states go to fs32 and the boundary fluxes to fb32. Vout (FP64)
-  // is written only where a later time step reads it (null otherwise).
+  // the stage input and of its result, and FP32 ghost states [5][bstride].
+  // Vout (FP64) is written only where a later time step reads it (null otherwise).
   const float* Vin32;
   float* Vout32;
   float* vg32;
-  // mixed forms, TVD-RK3: the stage whose result is the last stage's input
-  // (stage 2 of 3) also computes the next step's time step from the FP64
-  // primitives of that result, the ones the reference's calc_timestep reads
-  // (Solver.cpp:250): per cell into dt_next (local time stepping, else null)
-  // and the minimum into *dt_next_min (null: not this stage)
+  // fast forms, second order: where the stage kernel puts the cell-centre ghosts
+  // of its result, the next stage's (the other of two buffers; null: not needed)
+  double* vg_next;
+  float* vg_next32;
+  // fast forms: a stage that has the primitives the reference's calc_timestep
+  // reads (those of the last stage's input, Solver.cpp:250) also computes the
+  // next step's time step from them: the last stage from its input
+  // (dt_from_input; after the halo exchange of a split mesh), and the form with
+  // FP32 copies, which stages no FP64 primitives, under TVD-RK3 stage 2 of 3 from
+  // its FP64 result. Per cell into dt_next (local time stepping, else null) and
+  // the minimum into *dt_next_min (null: not this stage)
+  int dt_from_input;
   double* dt_next;
   unsigned long long* dt_next_min;
   const double* dS;  // [3][stride] projected areas (calc_Delta_S)
@@ -164,6 +173,10 @@ __device__ __forceinline__ void pdl_wait_previous() { asm volatile("griddepcontr
 // Once a case's ratchet is on, a cell's limiter value is the minimum of the
 // live value and the kept one, and is kept: it only tightens, so it settles
 // and the steady residual can converge (the live Barth limiter makes it stall).
+// Where another tile needs the cell's limiter in the same stage it evaluates the
+// same live value and takes the minimum with the kept one without writing it
+// (ratchet_seen): the same result whether it reads the kept value before or
+// after the owner's update, as that is the minimum with the same live value.
 __device__ __forceinline__ bool frozen_cell(const StageArgs& a, int c) {
   return a.case_frozen != nullptr && a.case_frozen[a.cell_case[c]] != 0;
 }
@@ -171,36 +184,22 @@ __device__ __forceinline__ bool ratchet_on(const StageArgs& a, int c) {
   return a.lim_ratchet != nullptr && a.lim_ratchet[a.cell_case[c]] != 0;
 }
 template <typename T>
-__device__ __forceinline__ T ratchet(const StageArgs& a, size_t at, T phi) {
-  T* keep;
+__device__ __forceinline__ T ratchet_seen(const StageArgs& a, size_t at, T phi) {
+  const volatile T* keep;
   if constexpr (sizeof(T) == 8) keep = a.phi_keep;
   else keep = a.phi_keep32;
-  const T v = (keep[at] < phi) ? keep[at] : phi;  // std::min(phi, kept)
+  const T v = keep[at];
+  return (v < phi) ? v : phi;  // std::min(phi, kept)
+}
+template <typename T>
+__device__ __forceinline__ T ratchet(const StageArgs& a, size_t at, T phi) {
+  volatile T* keep;
+  if constexpr (sizeof(T) == 8) keep = a.phi_keep;
+  else keep = a.phi_keep32;
+  const T v = ratchet_seen(a, at, phi);
   keep[at] = v;
   return v;
 }
-
-// The arrays the node kernels read and write, by arithmetic type: FP64 for
-// the FP64 form, the FP32 copies for the mixed form with FP32 copies
-// (primitives, ghosts, face states, boundary fluxes, optional dumps).
-template <typename T>
-struct StageIO;
-template <>
-struct StageIO<double> {
-  static __device__ __forceinline__ const double* vin(const StageArgs& a) { return a.Vin; }
-  static __device__ __forceinline__ const double* vg(const StageArgs& a) { return a.vg; }
-  static __device__ __forceinline__ double* fs(const StageArgs& a) { return a.fs; }
-  static __device__ __forceinline__ const double* fb(const StageArgs& a) { return a.fb; }
-  static __device__ __forceinline__ double* phi(const StageArgs& a) { return a.phi; }
-};
-template <>
-struct StageIO<float> {
-  static __device__ __forceinline__ const float* vin(const StageArgs& a) { return a.Vin32; }
-  static __device__ __forceinline__ const float* vg(const StageArgs& a) { return a.vg32; }
-  static __device__ __forceinline__ float* fs(const StageArgs& a) { return a.fs32; }
-  static __device__ __forceinline__ const float* fb(const StageArgs& a) { return a.fb32; }
-  static __device__ __forceinline__ float* phi(const StageArgs& a) { return a.phi32; }
-};
 
 // device scalars: the step's dt (minimum), the time, t_end, the dt last used,
 // and the next step's dt while the last stage computes it
@@ -512,15 +511,6 @@ __device__ __forceinline__ void warp_min_to(double v, unsigned long long* target
     atomicMin(target, (unsigned long long)__double_as_longlong(v));
 }
 
-// The next step's time step, computed by the FP64 form's last-stage gradient
-// kernel from the primitives it reads: those of the last stage input, which
-// the reference's calc_timestep reads (Solver.cpp:250).
-struct DtFuse {
-  double cfl;
-  double* dt_next;                  // per-cell dt of the next step (local time stepping) or null
-  unsigned long long* dt_min_bits;  // minimum over the cells (global time step)
-};
-
 // ---------------------------------------------------------------------------
 // Fast forms (FP64 with contraction, and mixed FP32): one thread per cell, the
 // cell's faces indexed by the vertex they face, geometry rebuilt from the
@@ -538,9 +528,9 @@ struct DtFuse {
 //   grad V . r_m = -1/2 sum_p (V_p + V_c) grad(lambda_p) . (centroid - P_m)
 //                = -1/2 sum_p (V_p + V_c) (1/4 - [p = m]) = 1/2 (V_m - M),
 //   M = mean of the four neighbours' values.
-// gradient_node_kernel therefore reads only the cell's own and its neighbours'
-// primitives: no vertices, normals, volume or face codes (agreement with the
-// reference form to round-off). A missing face (a boundary face no marker
+// So it takes only the cell's own and its neighbours' primitives: no vertices,
+// normals, volume or face codes (agreement with the reference form to
+// round-off). A missing face (a boundary face no marker
 // lists, FV_Grid.cpp:79-85) has S = r = 0 and names the cell itself; the sum
 // then runs over the listed faces, M = 1/4 sum_listed (V_p + V_c) - V_c.
 // The Barth limiter (Numerics.hpp:148-250) is
@@ -550,21 +540,6 @@ struct DtFuse {
 // smallest increment count, and with the formula above those are the largest
 // and the smallest neighbour value. One division per variable.
 // ---------------------------------------------------------------------------
-// Ask the memory system to bring a line into L2 without holding a register;
-// the later load of the same address then waits on an L2 hit, not on DRAM.
-__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
-
-// The own-cell rows the stage update reads (Uin, Un, the local dt).
-__device__ __forceinline__ void prefetch_update_rows(const StageArgs& a, int c, int st) {
-#pragma unroll
-  for (int k = 0; k < 5; k++) prefetch_l2(a.Uin + size_t(k) * st + c);
-  if (a.scheme != 0 && a.stage != 0) {
-#pragma unroll
-    for (int k = 0; k < 5; k++) prefetch_l2(a.Un + size_t(k) * st + c);
-  }
-  if (a.local_dt) prefetch_l2(a.dt_local + c);
-}
-
 // Node records are 4 values (x, y, z, pad) from a 256-byte aligned buffer, so
 // a record starts on 32 bytes (FP64) or 16 bytes (FP32): x and y come in one
 // 16-byte load (FP64), or the whole record in one (FP32).
@@ -609,119 +584,61 @@ __device__ __forceinline__ void face_normals(const T P[4][3], T S[4][3]) {
   face_normal<T, 3>(P, S[3]);
 }
 
-// Increments grad V . r_m of one variable from the neighbours' values minus
-// the cell's own, d_m, with limiter (barth): gr receives 1/2 (d_m - mean d),
-// and the limiter value is returned. n_missing faces are not listed (their d is
-// 0); shift is V_c (n_missing / 2), what they add to -M (0 for a closed cell).
+// max(v, 0) by the sign bit, off the FP64 pipe; FP32 minima and maxima are one
+// instruction. (A NaN anywhere in a cell's neighbourhood reaches the states
+// through the mean.)
+__device__ __forceinline__ double positive_part(double v) { return __double2hiint(v) < 0 ? 0.0 : v; }
+__device__ __forceinline__ float positive_part(float v) { return fmaxf(v, 0.f); }
+__device__ __forceinline__ void order_pair(double a, double b, double& lo, double& hi) {
+  const bool s = a < b;
+  lo = s ? a : b;
+  hi = s ? b : a;
+}
+__device__ __forceinline__ void order_pair(float a, float b, float& lo, float& hi) {
+  lo = fminf(a, b);
+  hi = fmaxf(a, b);
+}
+__device__ __forceinline__ double larger(double a, double b) { return a < b ? b : a; }
+__device__ __forceinline__ float larger(float a, float b) { return fmaxf(a, b); }
+
+// The limiter value of one variable (1 without a limiter) from the neighbours'
+// values minus the cell's own, d; *mean receives M - V_c, so the increment at
+// face m is 1/2 (d_m - *mean). none: bit m set where face m is not listed (its d
+// is 0 then); vc is the cell's own value. The operations are spelled out (fma)
+// so that every place that evaluates a cell gets the same bits.
 template <typename T>
-__device__ __forceinline__ T limited_increments(const T d[4], const int nb[4], int c, int n_missing, T shift, bool barth,
-                                                T gr[4]) {
-  const T mean = T(0.25) * ((d[0] + d[1]) + (d[2] + d[3])) - shift;
-#pragma unroll
-  for (int q = 0; q < 4; q++) gr[q] = T(0.5) * (d[q] - mean);
+__device__ __forceinline__ T limiter_value(const T d[4], unsigned none, T vc, bool barth, T* mean) {
+  const T sum = (d[0] + d[1]) + (d[2] + d[3]);
+  T mu = T(0.25) * sum;
+  // faces not listed add -1/2 V_c each to M - V_c
+  if (none) mu = fma(T(0.25), sum, T(-0.5) * T(__popc(none)) * vc);
+  *mean = mu;
   if (!barth) return T(1);
-  // extremes of two pairs, one comparison each
-  const bool s01 = d[0] < d[1], s23 = d[2] < d[3];
-  const T l0 = s01 ? d[0] : d[1], h0 = s01 ? d[1] : d[0], l1 = s23 ? d[2] : d[3], h1 = s23 ? d[3] : d[2];
-  const T dmax = rmax(h0, h1), dmin = rmin(l0, l1);
-  T ghi = T(0.5) * (dmax - mean), glo = T(0.5) * (dmin - mean);
-  if (n_missing) {  // listed faces only
-    ghi = glo = T(0);
+  T l0, h0, l1, h1;
+  order_pair(d[0], d[1], l0, h0);
+  order_pair(d[2], d[3], l1, h1);
+  const T dmax = larger(h0, h1), dmin = -larger(-l0, -l1);
+  T gh = dmax - mu, gl = mu - dmin;  // twice the largest and the smallest increment's size
+  if (none) {  // listed faces only
+    gh = gl = T(0);
 #pragma unroll
     for (int q = 0; q < 4; q++)
-      if (nb[q] != c) {
-        ghi = rmax(ghi, gr[q]);
-        glo = rmin(glo, gr[q]);
+      if (!(none >> q & 1)) {
+        gh = larger(gh, d[q] - mu);
+        gl = larger(gl, mu - d[q]);
       }
   }
   T An = T(1), Dn = T(1);  // best ratio so far, starting at 1
-  const T Ah = rmax(dmax, T(0)), Dh = ghi + Gas<T>::eps;   // V_max - V_c
-  const T Al = rmax(-dmin, T(0)), Dl = Gas<T>::eps - glo;  // V_c - V_min
-  if (ghi > T(0) && Ah < Dh) {
+  const T Ah = positive_part(dmax), Dh = fma(T(0.5), gh, Gas<T>::eps);   // V_max - V_c
+  const T Al = positive_part(-dmin), Dl = fma(T(0.5), gl, Gas<T>::eps);  // V_c - V_min
+  if (gh > T(0) && Ah < Dh) {
     An = Ah;
     Dn = Dh;
   }
-  const bool better = glo < T(0) && Al * Dn < An * Dl;
+  const bool better = gl > T(0) && Al * Dn < An * Dl;
   An = better ? Al : An;
   Dn = better ? Dl : Dn;
   return An * nr_rcp(Dn);
-}
-
-// kPipe: 0 one variable's loads at a time; 1 the next variable's loads in
-// flight during this one's arithmetic; 2 all five variables' loads issued
-// together before any arithmetic (one exposed memory latency instead of five,
-// at the cost of registers); 3 as 0, with the cell's own rows prefetched
-// into L2 first.
-// The body for one cell; vown receives the cell's own primitives.
-template <typename T, int kPipe>
-__device__ __forceinline__ void gradient_node_cell(const MeshView<T>& m, const StageArgs& a, int c, T vown[5]) {
-  const int st = m.stride;
-  const T* __restrict__ Vin = StageIO<T>::vin(a);
-  const T* __restrict__ Vg = StageIO<T>::vg(a);
-  T* __restrict__ fsc = StageIO<T>::fs(a) + c;  // this cell's column of the face states
-  int nb[4];
-#pragma unroll
-  for (int q = 0; q < 4; q++) nb[q] = checked_nb(m.nbvf[q * st + c], 0, m.n, m.nb, c, a.status);
-  // each face's row base and row stride (a cell's or a ghost's) chosen once,
-  // so a variable's neighbour load is one address computation
-  const T* qb[4];
-  int qs[4];
-#pragma unroll
-  for (int q = 0; q < 4; q++) {
-    const bool cell = nb[q] >= 0;
-    qb[q] = cell ? Vin + nb[q] : Vg + (-nb[q] - 1);
-    qs[q] = cell ? st : m.bstride;
-  }
-  auto fetch = [&](int k, T& vc, T vo[4]) {
-    vc = Vin[size_t(k) * st + c];
-#pragma unroll
-    for (int q = 0; q < 4; q++) vo[q] = qb[q][k * qs[q]];
-  };
-  if constexpr (kPipe == 3) {
-#pragma unroll
-    for (int k = 0; k < 5; k++) prefetch_l2(Vin + size_t(k) * st + c);
-  }
-  [[maybe_unused]] T vcN, voN[4];
-  [[maybe_unused]] T vcA[5], voA[5][4];
-  if constexpr (kPipe == 2) {
-#pragma unroll
-    for (int k = 0; k < 5; k++) fetch(k, vcA[k], voA[k]);
-  } else if (kPipe == 1) {
-    fetch(0, vcN, voN);
-  }
-  int n_missing = 0;
-#pragma unroll
-  for (int q = 0; q < 4; q++) n_missing += nb[q] == c;
-  const bool rat = a.barth && ratchet_on(a, c);
-  auto variable = [&](int k, T vc, const T vo[4]) {
-    vown[k] = vc;
-    T d[4], gr[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) d[q] = vo[q] - vc;
-    T phi = limited_increments(d, nb, c, n_missing, T(0.5) * T(n_missing) * vc, a.barth != 0, gr);
-    if (rat) phi = ratchet(a, size_t(k) * st + c, phi);
-#pragma unroll
-    for (int q = 0; q < 4; q++) fsc[size_t(q * 5 + k) * st] = fma(phi, gr[q], vc);
-    if (T* pdump = StageIO<T>::phi(a)) pdump[k * st + c] = phi;
-  };
-  if constexpr (kPipe == 2) {
-#pragma unroll
-    for (int k = 0; k < 5; k++) variable(k, vcA[k], voA[k]);
-  } else {
-#pragma unroll 1
-    for (int k = 0; k < 5; k++) {
-      T vc, vo[4];
-      if (kPipe == 1) {
-        vc = vcN;
-#pragma unroll
-        for (int q = 0; q < 4; q++) vo[q] = voN[q];
-        if (k < 4) fetch(k + 1, vcN, voN);  // next variable's loads overlap this one's arithmetic
-      } else {
-        fetch(k, vc, vo);
-      }
-      variable(k, vc, vo);
-    }
-  }
 }
 
 // CFL time step of one cell from its primitives with the fast forms'
@@ -732,37 +649,6 @@ __device__ __forceinline__ double dt_of_cell_fast(const double V[5], double dS0,
   const double cs = g * nr_rsqrt(g * V[0]);  // sqrt(gamma p / rho)
   const double sum = fma(fabs(V[3]) + cs, dS2, fma(fabs(V[2]) + cs, dS1, (fabs(V[1]) + cs) * dS0));
   return cfl * vol * nr_rcp(sum);
-}
-
-// kDt: also the next step's time step from the cell's own primitives, after
-// the gradient work (the FP64 form's last stage; the primitives are those of
-// the last stage input, which the reference's calc_timestep reads,
-// Solver.cpp:250; every thread reaches the block minimum).
-template <typename T, int kPipe, int kMinBlocks, bool kDt = false>
-__global__ void __launch_bounds__(128, kMinBlocks) gradient_node_kernel(MeshView<T> m, StageArgs a, DtFuse dtf) {
-  static_assert(!kDt || sizeof(T) == 8, "the fused time step is the FP64 form's");
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  pdl_launch_dependents();
-  pdl_wait_previous();
-  const bool in = c < m.n;
-  const bool active = in && !frozen_cell(a, c);
-  T vown[5];
-  if (active) gradient_node_cell<T, kPipe>(m, a, c, vown);
-  if constexpr (kDt) {
-    double dtc = DBL_MAX;
-    if (in) {
-      if (!active) {
-        if (dtf.dt_next) dtf.dt_next[c] = 0.0;  // a converged case keeps its state
-      } else {
-        const double d =
-            dt_of_cell_fast(vown, m.dS[c], m.dS[m.stride + c], m.dS[2 * m.stride + c], m.vol[c], dtf.cfl);
-        if (dtf.dt_next) dtf.dt_next[c] = d;
-        if (!(d > 0.0) && !isnan(d)) atomicOr(a.status, kErrDt);
-        if (d > 0.0) dtc = d;  // std::min skips NaN (comparisons with NaN are false)
-      }
-    }
-    warp_min_to(dtc, dtf.dt_min_bits);
-  }
 }
 
 // The Green-Gauss gradient itself (calc_green_gauss_gradient, Numerics.hpp:86-128)
@@ -805,25 +691,32 @@ __global__ void __launch_bounds__(128) gradient_field_kernel(MeshView<T> m, Stag
   }
 }
 
-// flux_node_kernel: flux balance and stage update of one cell per thread.
-// Each interior face's flux is evaluated with the reference's owner on the
-// left and the owner-to-neighbour unit normal, which both cells rebuild to the
-// same bits, so both add exactly opposite contributions; boundary faces add
-// the flux boundary_flux_kernel computed.
-template <typename T>
-struct FaceIn {
-  T s[5];      // this cell's face state, or the boundary flux
-  T x[5];      // the other side's face state
-  int kind;    // 0 no face, 1 interior (owner), 2 interior (neighbour side), 3 boundary
-};
+// The next step's time step of one cell from the primitives the reference's
+// calc_timestep reads (a.dt_next_min set): written where local time stepping
+// keeps it; returns its part of the minimum. A frozen cell keeps its state (dt 0).
+__device__ __forceinline__ double cell_next_dt(const StageArgs& a, int c, int st, const double V[5], double vol,
+                                               bool frozen) {
+  if (frozen) {
+    if (a.dt_next) a.dt_next[c] = 0.0;
+    return DBL_MAX;
+  }
+  const double d = dt_of_cell_fast(V, a.dS[c], a.dS[st + c], a.dS[2 * st + c], vol, a.cfl);
+  if (a.dt_next) a.dt_next[c] = d;
+  if (!(d > 0.0) && !isnan(d)) atomicOr(a.status, kErrDt);
+  return d > 0.0 ? d : DBL_MAX;  // std::min skips NaN (comparisons with NaN are false)
+}
 
-// Stage update of one cell from its flux balance R (TVD_RK3 Solver.cpp:103-133,
-// explicit_euler 83-101) in FP64, then the primitives of the new state
-// (set_primvars, SolverData.cpp:37-48), the optional dumps and the status.
-__device__ __forceinline__ void stage_update(const StageArgs& a, int c, int st, const double R[5], double vol) {
+// Stage update of one cell from its flux balance rs * R (TVD_RK3
+// Solver.cpp:103-133, explicit_euler 83-101) in FP64, then the primitives of the
+// new state (set_primvars, SolverData.cpp:37-48), the optional dumps and the
+// status. Returns the cell's part of the next step's minimum time step where
+// this stage computes it from its result, DBL_MAX otherwise. rs is a power of
+// two; Vn receives the new primitives.
+__device__ __forceinline__ double stage_update(const StageArgs& a, int c, int st, const double R[5], double rs,
+                                               double vol, double Vn[5]) {
   const double dt = a.local_dt ? a.dt_local[c] : stage_dt(a.scal);
   double Unew[5];
-  const double ivol = nr_rcp(vol);
+  const double ivol = rs * nr_rcp(vol);
   if (a.scheme == 0 || a.stage == 0) {
     const double qf = dt * ivol;
 #pragma unroll
@@ -841,150 +734,45 @@ __device__ __forceinline__ void stage_update(const StageArgs& a, int c, int st, 
 #pragma unroll
     for (int k = 0; k < 5; k++) Unew[k] = a.Uin[k * st + c];
   }
-  double Vn[5];
   cons_to_prim<double, false>(Unew, Vn);
-  bool finite = true;
+  // a non-finite R makes Unew non-finite (dt / vol is finite), so Unew alone is
+  // checked, by the exponents
+  int top = 0;
 #pragma unroll
   for (int k = 0; k < 5; k++) {
     a.Uout[k * st + c] = Unew[k];
-    if (a.Vout) a.Vout[k * st + c] = Vn[k];
-    if (a.Vout32) a.Vout32[k * st + c] = float(Vn[k]);
-    if (a.R) a.R[k * st + c] = R[k];
-    finite = finite && isfinite(R[k]) && isfinite(Unew[k]);
+    top = max(top, __double2hiint(Unew[k]) & 0x7fffffff);
+  }
+  if (a.Vout) {
+#pragma unroll
+    for (int k = 0; k < 5; k++) a.Vout[k * st + c] = Vn[k];
+  }
+  if (a.Vout32) {
+#pragma unroll
+    for (int k = 0; k < 5; k++) a.Vout32[k * st + c] = float(Vn[k]);
+  }
+  if (a.R) {
+#pragma unroll
+    for (int k = 0; k < 5; k++) a.R[k * st + c] = rs * R[k];
   }
   if (a.res_cell) a.res_cell[c] = R[0] * ivol;
-  if (!finite) atomicOr(a.status, kErrNonFinite);
+  if (top >= 0x7ff00000) atomicOr(a.status, kErrNonFinite);
   else if (!(Vn[0] > 0.0) || !(Vn[4] > 0.0)) atomicOr(a.status, kErrNonPhysical);
-  if (a.dt_next_min) {
-    // the next step's time step from this result's primitives; the minimum
-    // by one atomicMin on the bit pattern (exact for positive doubles),
-    // skipped when the value is not below the current minimum
-    const double d = (a.freeze && dt == 0.0) ? 0.0 : dt_of_cell_fast(Vn, a.dS[c], a.dS[st + c], a.dS[2 * st + c], vol, a.cfl);
-    if (a.dt_next) a.dt_next[c] = d;
-    if (!(a.freeze && dt == 0.0)) {
-      if (!(d > 0.0) && !isnan(d)) atomicOr(a.status, kErrDt);
-      if (d > 0.0 &&
-          d < __longlong_as_double(static_cast<long long>(*reinterpret_cast<volatile unsigned long long*>(a.dt_next_min))))
-        atomicMin(a.dt_next_min, (unsigned long long)__double_as_longlong(d));
-    }
-  }
-}
-
-// kPipe: 0 one face's loads at a time, 1 the next face's loads in flight
-// during this face's flux, 2 all four faces' loads issued together, 3 as 0
-// with the cell's own face states and update rows prefetched into L2 first.
-template <typename T, int kPipe, int kMinBlocks>
-__global__ void __launch_bounds__(128, kMinBlocks) flux_node_kernel(MeshView<T> m, StageArgs a) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  pdl_launch_dependents();
-  pdl_wait_previous();
-  if (c >= m.n) return;
-  if (frozen_cell(a, c)) {
-    if (a.dt_next_min && a.dt_next) a.dt_next[c] = 0.0;  // a converged case keeps its state
-    return;
-  }
-  const int st = m.stride;
-  const bool second = a.second_order != 0;
-  const T* __restrict__ fsb = StageIO<T>::fs(a);
-  const T* __restrict__ Vin = StageIO<T>::vin(a);
-  const T* __restrict__ fb = StageIO<T>::fb(a);
-  const int code = m.gcode[c];
-  int ns[4];
-#pragma unroll
-  for (int q = 0; q < 4; q++) ns[q] = checked_nb(m.nbsf[q * st + c], 2, m.n, m.nb, c << 2 | q, a.status);
-  auto fetch = [&](int q, FaceIn<T>& in) {
-    const int bits = code >> (3 * q);
-    if ((bits & 1) == 0) {
-      in.kind = 0;
-    } else if (ns[q] < 0) {
-      in.kind = 3;
-      const int b = -ns[q] - 1;
-#pragma unroll
-      for (int k = 0; k < 5; k++) in.s[k] = fb[k * m.bstride + b];
-    } else {
-      const int o = ns[q] >> 2, q2 = ns[q] & 3;
-      in.kind = (bits & 4) ? 2 : 1;
-#pragma unroll
-      for (int k = 0; k < 5; k++) {
-        in.s[k] = second ? fsb[(q * 5 + k) * st + c] : Vin[k * st + c];
-        in.x[k] = second ? fsb[(q2 * 5 + k) * st + o] : Vin[k * st + o];
-      }
-    }
-  };
-  if constexpr (kPipe == 3) {
-    if (second) {
-#pragma unroll
-      for (int r = 0; r < 20; r++) prefetch_l2(fsb + size_t(r) * st + c);
-    }
-    prefetch_update_rows(a, c, st);
-  }
-  [[maybe_unused]] FaceIn<T> nxt;
-  [[maybe_unused]] FaceIn<T> all[4];
-  if constexpr (kPipe == 2) {
-#pragma unroll
-    for (int q = 0; q < 4; q++) fetch(q, all[q]);
-  } else if (kPipe == 1) {
-    fetch(0, nxt);
-  }
-  T S[4][3];
-  {
-    T P[4][3];
-    load_vertices(m, c, P, a.status);
-    face_normals(P, S);
-  }
-  // the flux balance in FP64 (FP64 form); the FP32 form sums its FP32 fluxes
-  // in FP32 and hands the sum to the FP64 update
-  using Acc = typename std::conditional<sizeof(T) == 8, double, float>::type;
-  Acc R[5] = {Acc(0), Acc(0), Acc(0), Acc(0), Acc(0)};
-#pragma unroll
-  for (int q = 0; q < 4; q++) {
-    FaceIn<T> cur;
-    if constexpr (kPipe == 2) {
-      cur = all[q];
-    } else if (kPipe == 1) {
-      cur = nxt;
-      if (q < 3) fetch(q + 1, nxt);  // next face's loads overlap this face's flux
-    } else {
-      fetch(q, cur);
-    }
-    if (cur.kind == 3) {
-#pragma unroll
-      for (int k = 0; k < 5; k++) R[k] -= Acc(cur.s[k]);
-    } else if (cur.kind != 0) {
-      const int bits = code >> (3 * q);
-      const bool own = cur.kind == 1;
-      // owner-to-neighbour normal: this cell's outward normal on the owner side
-      const bool flip = own ? (bits & 2) != 0 : (bits & 2) == 0;
-      const T a2 = (S[q][0] * S[q][0] + S[q][1] * S[q][1]) + S[q][2] * S[q][2];
-      const T inv = nr_rsqrt(a2);  // 1 / |S|
-      const T area = a2 * inv;
-      const T sg = flip ? -inv : inv;
-      const T nh[3] = {S[q][0] * sg, S[q][1] * sg, S[q][2] * sg};
-      T Fl[5];
-      if (own) rusanov_fast<T>(cur.s, cur.x, nh, area, Fl);
-      else rusanov_fast<T>(cur.x, cur.s, nh, area, Fl);
-#pragma unroll
-      for (int k = 0; k < 5; k++) R[k] = own ? R[k] - Acc(Fl[k]) : R[k] + Acc(Fl[k]);
-    }
-  }
-  const double Rd[5] = {double(R[0]), double(R[1]), double(R[2]), double(R[3]), double(R[4])};
-  stage_update(a, c, st, Rd, m.vol[c]);
+  return a.dt_next_min && !a.dt_from_input ? cell_next_dt(a, c, st, Vn, vol, a.freeze && dt == 0.0) : DBL_MAX;
 }
 
 // ---------------------------------------------------------------------------
-// Boundary faces. ghost_kernel: the cell-centre ghost state of every boundary
-// face (set_constant_ghost_values, Solver.cpp:300-330), read by the gradient
-// kernel like a neighbour's primitives. boundary_flux_kernel: the flux through
-// every boundary face, from the owner's reconstructed face state and the ghost
-// built from that state (Solver.cpp:197-229), read by the flux kernel at the
-// face's slot. One thread per boundary face; the hot kernels carry no
-// boundary-condition code.
+// Boundary faces of the reference-order form. ghost_kernel: the cell-centre ghost
+// state of every boundary face (set_constant_ghost_values, Solver.cpp:300-330),
+// read by the gradient kernel like a neighbour's primitives.
+// boundary_flux_kernel: the flux through every boundary face, from the owner's
+// reconstructed face state and the ghost built from that state
+// (Solver.cpp:197-229), read by the flux kernel at the face's slot. One thread
+// per boundary face; the other kernels carry no boundary-condition code.
 // ---------------------------------------------------------------------------
-template <typename T, bool kRef>
+template <typename T>
 __global__ void __launch_bounds__(256) ghost_kernel(MeshView<T> m, StageArgs a) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  pdl_launch_dependents();
-  pdl_wait_previous();
   if (b >= m.nb) return;
   const int c = checked(m.b_cell[b], m.n, a.status), f = checked(m.b_face[b], m.n_faces, a.status);
   const int F = m.n_faces, st = m.stride;
@@ -994,40 +782,25 @@ __global__ void __launch_bounds__(256) ghost_kernel(MeshView<T> m, StageArgs a) 
   const T nh[3] = {m.nhat[f], m.nhat[F + f], m.nhat[2 * F + f]};
   ghost_state<T>(m.patches[checked(m.b_patch[b], m.n_patches, a.status)], V, nh, G);
 #pragma unroll
-  for (int k = 0; k < 5; k++) {
-    a.vg[k * m.bstride + b] = G[k];
-  }
+  for (int k = 0; k < 5; k++) a.vg[k * m.bstride + b] = G[k];
 }
 
-template <typename T, bool kRef>
+template <typename T>
 __global__ void __launch_bounds__(256) boundary_flux_kernel(MeshView<T> m, StageArgs a) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  pdl_launch_dependents();
-  pdl_wait_previous();
   if (b >= m.nb) return;
-  const int c = checked(m.b_cell[b], m.n, a.status), q = checked(m.b_fs[b], 4, a.status),
+  const int c = checked(m.b_cell[b], m.n, a.status), q = checked(m.b_slot[b], 4, a.status),
             f = checked(m.b_face[b], m.n_faces, a.status);
   const int F = m.n_faces, st = m.stride;
   T VL[5], VR[5];
 #pragma unroll
-  for (int k = 0; k < 5; k++) {
-    if (a.second_order) {
-      VL[k] = a.fs[(q * 5 + k) * st + c];
-    } else {
-      VL[k] = ld_v<T>(a, k * st + c);
-    }
-  }
+  for (int k = 0; k < 5; k++) VL[k] = a.second_order ? a.fs[(q * 5 + k) * st + c] : ld_v<T>(a, k * st + c);
   const T nh[3] = {m.nhat[f], m.nhat[F + f], m.nhat[2 * F + f]};
   ghost_state<T>(m.patches[checked(m.b_patch[b], m.n_patches, a.status)], VL, nh, VR);
-  T Fl[5];
-  if constexpr (kRef) {
-    T UL[5], UR[5];
-    prim_to_cons<T, kRef>(VL, UL);
-    prim_to_cons<T, kRef>(VR, UR);
-    rusanov_ref<T>(UL, UR, nh, m.area[f], Fl);
-  } else {
-    rusanov_fast<T>(VL, VR, nh, m.area[f], Fl);
-  }
+  T Fl[5], UL[5], UR[5];
+  prim_to_cons<T, true>(VL, UL);
+  prim_to_cons<T, true>(VR, UR);
+  rusanov_ref<T>(UL, UR, nh, m.area[f], Fl);
 #pragma unroll
   for (int k = 0; k < 5; k++) a.fb[k * m.bstride + b] = Fl[k];
 }

@@ -1,9 +1,9 @@
-// Kernels with reciprocals and fused multiply-adds (FP64), and the
-// mixed-precision form (FP32 face work in difference variables, FP64 state,
-// primitives, ghosts, boundary fluxes and update).
+// Launchers of the forms with reciprocals and fused multiply-adds: FP64, and the
+// mixed forms (FP32 face work; FP64 state, ghosts, boundary fluxes and update).
+#include <type_traits>
 #include <utility>
 
-#include "kernels_mixed.cuh"
+#include "kernels_copy.cuh"
 #include "launch.hpp"
 
 namespace nf {
@@ -31,10 +31,11 @@ static inline int grid_for(int n, int block) { return (n + block - 1) / block; }
 // before reading its results, pdl_wait_previous). Captured into the step's
 // CUDA graph as a programmatic dependency.
 template <typename... P, typename... A>
-static void launch_pdl(void (*kernel)(P...), int grid, int block, cudaStream_t stream, A&&... args) {
+static void launch_pdl(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t stream, A&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(unsigned(grid));
   cfg.blockDim = dim3(unsigned(block));
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -44,169 +45,142 @@ static void launch_pdl(void (*kernel)(P...), int grid, int block, cudaStream_t s
   cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
-// one thread per cell, at most 128 threads per block (the kernels' launch bounds)
-static inline int fast_block(int b) { return b > 128 ? 128 : b; }
+// ---- the stage kernel ----
+// Threads an SM should hold, which caps a thread's registers: three blocks of 256
+// at 80 registers (also what their shared memory allows), four at 64 for the form
+// with FP32 copies. Per launch at 3.1M tets: FP64 455 us with two blocks at 128
+// registers, 369 us with three; FP32 copies 291 us with three, 251 us with four;
+// difference form 374 us with three, 408 us with four (spills).
+template <int kForm>
+constexpr int kThreadsPerSm = kForm == kFormCopy ? 1024 : 768;
 
-// Variants (the tuner times them): 0 plain, 1 software-pipelined, 2 plain
-// with registers capped for at least kCap resident 128-thread blocks per SM
-// (6 for FP64, 8 for FP32), 3 pipelined with the same cap, 4 and 5 the same
-// with a tighter cap (7 / 9 blocks), 6 and 7 with every load issued before the
-// arithmetic (kPipe 2), uncapped and capped for kCap3 blocks (4 / 5), 8 and 9
-// plain with the cell's own rows prefetched into L2 (kPipe 3), capped as 2
-// and 4. (Prefetching the neighbours' rows as well measured slower.)
-template <typename T>
-constexpr int kCap = sizeof(T) == 8 ? 6 : 8;
-template <typename T>
-constexpr int kCap2 = sizeof(T) == 8 ? 7 : 9;
-template <typename T>
-constexpr int kCap3 = sizeof(T) == 8 ? 4 : 5;
-#define NF_NODE_DISPATCH(KERNEL, T, m, a, l)                                                       \
-  do {                                                                                              \
-    const int b = fast_block(l.block);                                                             \
-    const int g = grid_for(m.n, b);                                                                \
-    switch (l.variant) {                                                                            \
-      case 1: launch_pdl(KERNEL<T, 1, 1>, g, b, l.stream, m, a); break;                                 \
-      case 2: launch_pdl(KERNEL<T, 0, kCap<T>>, g, b, l.stream, m, a); break;                           \
-      case 3: launch_pdl(KERNEL<T, 1, kCap<T>>, g, b, l.stream, m, a); break;                           \
-      case 4: launch_pdl(KERNEL<T, 0, kCap2<T>>, g, b, l.stream, m, a); break;                          \
-      case 5: launch_pdl(KERNEL<T, 1, kCap2<T>>, g, b, l.stream, m, a); break;                          \
-      case 6: launch_pdl(KERNEL<T, 2, 1>, g, b, l.stream, m, a); break;                                 \
-      case 7: launch_pdl(KERNEL<T, 2, kCap3<T>>, g, b, l.stream, m, a); break;                          \
-      case 8: launch_pdl(KERNEL<T, 3, kCap<T>>, g, b, l.stream, m, a); break;                           \
-      case 9: launch_pdl(KERNEL<T, 3, kCap2<T>>, g, b, l.stream, m, a); break;                          \
-      default: launch_pdl(KERNEL<T, 0, 1>, g, b, l.stream, m, a); break;                                \
-    }                                                                                               \
-  } while (0)
+// f(kernel, form, row length) for the form, tile size and mode
+template <typename Fn>
+static void with_stage_kernel(int form, int tile, int mode, Fn&& f) {
+  auto order = [&](auto frm, auto tc, auto row) {
+    constexpr int kF = decltype(frm)::value, kT = decltype(tc)::value, kR = decltype(row)::value;
+    constexpr int kB = kThreadsPerSm<kF> / kT;
+    if (mode == kModeFirst) f(stage_kernel<kF, kT, kR, kB, kModeFirst>, frm, row);
+    else if (mode == kModePlain) f(stage_kernel<kF, kT, kR, kB, kModePlain>, frm, row);
+    else if (mode == kModeGhosts) f(stage_kernel<kF, kT, kR, kB, kModeGhosts>, frm, row);
+    else f(stage_kernel<kF, kT, kR, kB, kModeGeneral>, frm, row);
+  };
+  auto size = [&](auto frm) {
+    using std::integral_constant;
+    // 256 threads: the largest tile whose lists fit three times in an SM's shared
+    // memory (at 3.1M tets FP64 369 us a launch, 379 us at 192, 413 us at 160,
+    // 520 us or more at 128). Meshes whose tiles touch more than its rows hold
+    // (thin or badly ordered ones) take 128 with longer rows, then 64, whose rows
+    // hold whatever its cells can touch (17 values a cell).
+    if (tile == 256) order(frm, integral_constant<int, 256>(), integral_constant<int, 6 * 256>());
+    else if (tile == 128) order(frm, integral_constant<int, 128>(), integral_constant<int, 8 * 128>());
+    else order(frm, integral_constant<int, 64>(), integral_constant<int, 17 * 64>());
+  };
+  if (form == kFormFp64) size(std::integral_constant<int, kFormFp64>());
+  else if (form == kFormDelta) size(std::integral_constant<int, kFormDelta>());
+  else size(std::integral_constant<int, kFormCopy>());
+}
 
-// the gradient kernel's variants, with and without the next step's time step
-#define NF_GRAD_DISPATCH(KDT)                                                                       \
-  do {                                                                                              \
-    const int b = fast_block(l.block);                                                             \
-    const int g = grid_for(m.n, b);                                                                \
-    switch (l.variant) {                                                                            \
-      case 1: launch_pdl(gradient_node_kernel<double, 1, 1, KDT>, g, b, l.stream, m, a, d); break;       \
-      case 2: launch_pdl(gradient_node_kernel<double, 0, kCap<double>, KDT>, g, b, l.stream, m, a, d); break; \
-      case 3: launch_pdl(gradient_node_kernel<double, 1, kCap<double>, KDT>, g, b, l.stream, m, a, d); break; \
-      case 4: launch_pdl(gradient_node_kernel<double, 0, kCap2<double>, KDT>, g, b, l.stream, m, a, d); break; \
-      case 5: launch_pdl(gradient_node_kernel<double, 1, kCap2<double>, KDT>, g, b, l.stream, m, a, d); break; \
-      case 6: launch_pdl(gradient_node_kernel<double, 2, 1, KDT>, g, b, l.stream, m, a, d); break;       \
-      case 7: launch_pdl(gradient_node_kernel<double, 2, kCap3<double>, KDT>, g, b, l.stream, m, a, d); break; \
-      case 8: launch_pdl(gradient_node_kernel<double, 3, kCap<double>, KDT>, g, b, l.stream, m, a, d); break; \
-      case 9: launch_pdl(gradient_node_kernel<double, 3, kCap2<double>, KDT>, g, b, l.stream, m, a, d); break; \
-      default: launch_pdl(gradient_node_kernel<double, 0, 1, KDT>, g, b, l.stream, m, a, d); break;      \
-    }                                                                                               \
-  } while (0)
+size_t stage_smem(int form, const Tiles& t, bool second) {
+  size_t bytes = 0;
+  with_stage_kernel(form, t.tile, second ? kModePlain : kModeFirst, [&](auto, auto frm, auto row) {
+    constexpr int kR = decltype(row)::value;
+    const bool fits = (second ? t.max_staged2 : t.max_staged1) <= kR && (!second || t.max_states <= kR);
+    bytes = fits ? tile_smem_bytes<decltype(frm)::value, kR>(t.max_nodes) : 0;
+  });
+  return bytes;
+}
+cudaError_t stage_setup(int form, int tile, int mode, int max_smem, size_t smem, int* blocks) {
+  cudaError_t e = cudaSuccess;
+  with_stage_kernel(form, tile, mode, [&](auto k, auto, auto) {
+    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, k, tile, smem);
+  });
+  return e;
+}
+void launch_stage(int form, int tile, int mode, const MeshView<double>& m, const TileView& tv, const StageArgs& a,
+                  size_t smem, cudaStream_t st) {
+  with_stage_kernel(form, tile, mode, [&](auto k, auto, auto) { launch_pdl(k, tv.n_tiles, tile, smem, st, m, tv, a); });
+}
+// The form with FP32 copies under the Barth limiter: launch variants the tuner
+// times. 0 plain, 1 software-pipelined, 2 and 3 the same with registers capped
+// for 8 resident 128-thread blocks an SM, 4 and 5 for 9, 6 and 7 with every load
+// issued before the arithmetic, uncapped and capped for 5, 8 and 9 plain with the
+// cell's own rows prefetched into L2, capped as 2 and 4.
+template <typename Fn>
+static void with_variant(int variant, Fn&& f) {
+  using std::integral_constant;
+  auto go = [&](auto pipe, auto blocks) { f(pipe, blocks); };
+  using P0 = integral_constant<int, 0>;
+  using P1 = integral_constant<int, 1>;
+  using P2 = integral_constant<int, 2>;
+  using P3 = integral_constant<int, 3>;
+  switch (variant) {
+    case 1: go(P1(), integral_constant<int, 1>()); break;
+    case 2: go(P0(), integral_constant<int, 8>()); break;
+    case 3: go(P1(), integral_constant<int, 8>()); break;
+    case 4: go(P0(), integral_constant<int, 9>()); break;
+    case 5: go(P1(), integral_constant<int, 9>()); break;
+    case 6: go(P2(), integral_constant<int, 1>()); break;
+    case 7: go(P2(), integral_constant<int, 5>()); break;
+    case 8: go(P3(), integral_constant<int, 8>()); break;
+    case 9: go(P3(), integral_constant<int, 9>()); break;
+    default: go(P0(), integral_constant<int, 1>()); break;
+  }
+}
+void launch_gradient_copy(const MeshView<float>& m, const StageArgs& a, Launch l, int variant) {
+  const int b = l.block > 128 ? 128 : l.block;
+  with_variant(variant, [&](auto pipe, auto blocks) {
+    launch_pdl(gradient_copy_kernel<decltype(pipe)::value, decltype(blocks)::value>, grid_for(m.n, b), b, 0, l.stream,
+               m, a);
+  });
+}
+void launch_flux_copy(const MeshView<float>& m, const StageArgs& a, Launch l, int variant) {
+  const int b = l.block > 128 ? 128 : l.block;
+  with_variant(variant, [&](auto pipe, auto blocks) {
+    launch_pdl(flux_copy_kernel<decltype(pipe)::value, decltype(blocks)::value>, grid_for(m.n, b), b, 0, l.stream, m, a);
+  });
+}
+void launch_bflux_copy(const MeshView<double>& m, const TileView& tv, const StageArgs& a, Launch l) {
+  if (m.nb > 0) launch_pdl(boundary_flux_copy_kernel, grid_for(m.nb, l.block), l.block, 0, l.stream, m, tv, a);
+}
+void launch_gradient_field(int form, const MeshView<double>& m, const MeshView<float>& m32, const StageArgs& a,
+                           cudaStream_t st) {
+  const int g = grid_for(m.n, 128);
+  if (form == kFormFp64) gradient_field_kernel<double, double><<<g, 128, 0, st>>>(m, a, a.Vin, a.vg, a.grad);
+  else if (form == kFormDelta) gradient_field_kernel<float, double><<<g, 128, 0, st>>>(m32, a, a.Vin, a.vg, a.grad32);
+  else gradient_field_kernel<float, float><<<g, 128, 0, st>>>(m32, a, a.Vin32, a.vg32, a.grad32);
+}
 
-void launch_gradient_fast(const MeshView<double>& m, const StageArgs& a, const DtFuse* dt, Launch l) {
-  const DtFuse d = dt ? *dt : DtFuse{0.0, nullptr, nullptr};
-  if (dt) NF_GRAD_DISPATCH(true);
-  else NF_GRAD_DISPATCH(false);
-  if (a.grad) gradient_field_kernel<double, double><<<grid_for(m.n, 128), 128, 0, l.stream>>>(m, a, a.Vin, a.vg, a.grad);
-}
-#undef NF_GRAD_DISPATCH
-void launch_flux_fast(const MeshView<double>& m, const StageArgs& a, Launch l) {
-  NF_NODE_DISPATCH(flux_node_kernel, double, m, a, l);
-}
-// mixed form (difference variables, kernels_mixed.cuh)
-#define NF_DELTA_DISPATCH(KERNEL, m, a, l)                                                         \
-  do {                                                                                              \
-    const int b = fast_block(l.block);                                                             \
-    const int g = grid_for(m.n, b);                                                                \
-    switch (l.variant) {                                                                            \
-      case 1: launch_pdl(KERNEL<1, 1>, g, b, l.stream, m, a); break;                                    \
-      case 2: launch_pdl(KERNEL<0, kCap<float>>, g, b, l.stream, m, a); break;                          \
-      case 3: launch_pdl(KERNEL<1, kCap<float>>, g, b, l.stream, m, a); break;                          \
-      case 4: launch_pdl(KERNEL<0, kCap2<float>>, g, b, l.stream, m, a); break;                         \
-      case 5: launch_pdl(KERNEL<1, kCap2<float>>, g, b, l.stream, m, a); break;                         \
-      case 6: launch_pdl(KERNEL<2, 1>, g, b, l.stream, m, a); break;                                    \
-      case 7: launch_pdl(KERNEL<2, kCap3<float>>, g, b, l.stream, m, a); break;                         \
-      case 8: launch_pdl(KERNEL<3, kCap<float>>, g, b, l.stream, m, a); break;                          \
-      case 9: launch_pdl(KERNEL<3, kCap2<float>>, g, b, l.stream, m, a); break;                         \
-      default: launch_pdl(KERNEL<0, 1>, g, b, l.stream, m, a); break;                                   \
-    }                                                                                               \
-  } while (0)
-
-void launch_gradient_mixed(const MeshView<float>& m, const StageArgs& a, Launch l) {
-  NF_DELTA_DISPATCH(gradient_delta_kernel, m, a, l);
-  if (a.grad32) gradient_field_kernel<float, double><<<grid_for(m.n, 128), 128, 0, l.stream>>>(m, a, a.Vin, a.vg, a.grad32);
-}
-void launch_flux_mixed(const MeshView<float>& m, const StageArgs& a, Launch l) {
-  NF_DELTA_DISPATCH(flux_delta_kernel, m, a, l);
-}
-// The mixed form with FP32 copies: ghost states and boundary fluxes computed
-// in FP64 from the FP32 primitives or face states (boundary faces are a few
-// percent of the faces) and stored in FP32 for the FP32 node kernels.
-__global__ void __launch_bounds__(256) ghost32_kernel(MeshView<double> m, StageArgs a) {
+// The cell-centre ghost state of every boundary face from the stage input's
+// primitives (set_constant_ghost_values, Solver.cpp:300-330), where the previous
+// stage kernel did not leave it. kCopy: from the FP32 primitives, computed in
+// FP64 (boundary faces are a few percent of the faces), stored in FP32, with the
+// powers as ever (kernels_copy.cuh says why).
+template <bool kCopy>
+__global__ void __launch_bounds__(256) ghost_kernel_fast(MeshView<double> m, TileView tv, StageArgs a) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   pdl_launch_dependents();
   pdl_wait_previous();
   if (b >= m.nb) return;
-  const int c = checked(m.b_cell[b], m.n, a.status), f = checked(m.b_face[b], m.n_faces, a.status);
-  const int F = m.n_faces, st = m.stride;
+  const int2 ref = tv.b_ref[b];
+  const double4 geo = tv.b_geo[b];
+  const int c = checked(ref.x >> 2, m.n, a.status), st = m.stride;
+  const double nh[3] = {geo.x, geo.y, geo.z};
   double V[5], G[5];
 #pragma unroll
-  for (int k = 0; k < 5; k++) V[k] = double(a.Vin32[k * st + c]);
-  const double nh[3] = {m.nhat[f], m.nhat[F + f], m.nhat[2 * F + f]};
-  ghost_state<double>(m.patches[checked(m.b_patch[b], m.n_patches, a.status)], V, nh, G);
+  for (int k = 0; k < 5; k++) V[k] = kCopy ? double(a.Vin32[k * st + c]) : a.Vin[k * st + c];
+  ghost_state<double, kCopy>(m.patches[checked(ref.y, m.n_patches, a.status)], V, nh, G);
 #pragma unroll
-  for (int k = 0; k < 5; k++) a.vg32[k * m.bstride + b] = float(G[k]);
-}
-
-__global__ void __launch_bounds__(256) boundary_flux32_kernel(MeshView<double> m, StageArgs a) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  pdl_launch_dependents();
-  pdl_wait_previous();
-  if (b >= m.nb) return;
-  const int c = checked(m.b_cell[b], m.n, a.status), q = checked(m.b_fs[b], 4, a.status),
-            f = checked(m.b_face[b], m.n_faces, a.status);
-  const int F = m.n_faces, st = m.stride;
-  double VL[5], VR[5];
-#pragma unroll
-  for (int k = 0; k < 5; k++) VL[k] = double(a.second_order ? a.fs32[(q * 5 + k) * st + c] : a.Vin32[k * st + c]);
-  const double nh[3] = {m.nhat[f], m.nhat[F + f], m.nhat[2 * F + f]};
-  ghost_state<double>(m.patches[checked(m.b_patch[b], m.n_patches, a.status)], VL, nh, VR);
-  double Fl[5];
-  rusanov_fast<double>(VL, VR, nh, m.area[f], Fl);
-#pragma unroll
-  for (int k = 0; k < 5; k++) a.fb32[k * m.bstride + b] = float(Fl[k]);
-}
-
-// mixed form with FP32 copies: the node kernels in FP32 (no fused time step)
-void launch_gradient_m32(const MeshView<float>& m, const StageArgs& a, Launch l) {
-  const DtFuse d{0.0, nullptr, nullptr};
-  const int b = fast_block(l.block);
-  const int g = grid_for(m.n, b);
-  switch (l.variant) {
-    case 1: launch_pdl(gradient_node_kernel<float, 1, 1, false>, g, b, l.stream, m, a, d); break;
-    case 2: launch_pdl(gradient_node_kernel<float, 0, kCap<float>, false>, g, b, l.stream, m, a, d); break;
-    case 3: launch_pdl(gradient_node_kernel<float, 1, kCap<float>, false>, g, b, l.stream, m, a, d); break;
-    case 4: launch_pdl(gradient_node_kernel<float, 0, kCap2<float>, false>, g, b, l.stream, m, a, d); break;
-    case 5: launch_pdl(gradient_node_kernel<float, 1, kCap2<float>, false>, g, b, l.stream, m, a, d); break;
-    case 6: launch_pdl(gradient_node_kernel<float, 2, 1, false>, g, b, l.stream, m, a, d); break;
-    case 7: launch_pdl(gradient_node_kernel<float, 2, kCap3<float>, false>, g, b, l.stream, m, a, d); break;
-    case 8: launch_pdl(gradient_node_kernel<float, 3, kCap<float>, false>, g, b, l.stream, m, a, d); break;
-    case 9: launch_pdl(gradient_node_kernel<float, 3, kCap2<float>, false>, g, b, l.stream, m, a, d); break;
-    default: launch_pdl(gradient_node_kernel<float, 0, 1, false>, g, b, l.stream, m, a, d); break;
+  for (int k = 0; k < 5; k++) {
+    if constexpr (kCopy) a.vg32[k * m.bstride + b] = float(G[k]);
+    else a.vg[k * m.bstride + b] = G[k];
   }
-  if (a.grad32) gradient_field_kernel<float, float><<<g, b, 0, l.stream>>>(m, a, a.Vin32, a.vg32, a.grad32);
 }
-void launch_flux_m32(const MeshView<float>& m, const StageArgs& a, Launch l) {
-  NF_NODE_DISPATCH(flux_node_kernel, float, m, a, l);
-}
-void launch_ghost_m32(const MeshView<double>& m, const StageArgs& a, Launch l) {
-  if (m.nb > 0) launch_pdl(ghost32_kernel, grid_for(m.nb, l.block), l.block, l.stream, m, a);
-}
-void launch_bflux_m32(const MeshView<double>& m, const StageArgs& a, Launch l) {
-  if (m.nb > 0) launch_pdl(boundary_flux32_kernel, grid_for(m.nb, l.block), l.block, l.stream, m, a);
-}
-void launch_ghost_fast(const MeshView<double>& m, const StageArgs& a, Launch l) {
-  if (m.nb > 0) launch_pdl(ghost_kernel<double, false>, grid_for(m.nb, l.block), l.block, l.stream, m, a);
-}
-void launch_bflux_fast(const MeshView<double>& m, const StageArgs& a, Launch l) {
-  if (m.nb > 0) launch_pdl(boundary_flux_kernel<double, false>, grid_for(m.nb, l.block), l.block, l.stream, m, a);
-}
-void launch_bflux_mixed(const MeshView<double>& m, const StageArgs& a, Launch l) {
-  if (m.nb > 0) launch_pdl(boundary_flux_delta_kernel, grid_for(m.nb, l.block), l.block, l.stream, m, a);
+void launch_ghost(int form, const MeshView<double>& m, const TileView& tv, const StageArgs& a, Launch l) {
+  if (m.nb == 0) return;
+  auto* k = form == kFormCopy ? ghost_kernel_fast<true> : ghost_kernel_fast<false>;
+  launch_pdl(k, grid_for(m.nb, l.block), l.block, 0, l.stream, m, tv, a);
 }
 __global__ void fastmath_kernel(const double* x, int n, double* rcp, double* rsq) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;

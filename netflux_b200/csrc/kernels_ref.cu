@@ -29,10 +29,10 @@ void launch_flux_ref(const MeshView<double>& m, const StageArgs& a, Launch l) {
   flux_update_kernel<double, true><<<grid_for(4 * m.n, l.block), l.block, 0, l.stream>>>(m, a);
 }
 void launch_ghost_ref(const MeshView<double>& m, const StageArgs& a, Launch l) {
-  if (m.nb > 0) ghost_kernel<double, true><<<grid_for(m.nb, l.block), l.block, 0, l.stream>>>(m, a);
+  if (m.nb > 0) ghost_kernel<double><<<grid_for(m.nb, l.block), l.block, 0, l.stream>>>(m, a);
 }
 void launch_bflux_ref(const MeshView<double>& m, const StageArgs& a, Launch l) {
-  if (m.nb > 0) boundary_flux_kernel<double, true><<<grid_for(m.nb, l.block), l.block, 0, l.stream>>>(m, a);
+  if (m.nb > 0) boundary_flux_kernel<double><<<grid_for(m.nb, l.block), l.block, 0, l.stream>>>(m, a);
 }
 void launch_timestep(const MeshView<double>& m, const DtArgs& a, Launch l) {
   timestep_kernel<true><<<grid_for(m.n, l.block), l.block, 0, l.stream>>>(m, a);

@@ -12,7 +12,6 @@ namespace nf {
 struct Launch {
   int block;
   cudaStream_t stream;
-  int variant = 0;  // fast kernels: bit 0 software-pipelined, bit 1 registers capped for occupancy
 };
 
 // reference-order FP64 (kernels_ref.cu)
@@ -23,25 +22,25 @@ void launch_bflux_ref(const MeshView<double>& m, const StageArgs& a, Launch l);
 void launch_timestep(const MeshView<double>& m, const DtArgs& a, Launch l);
 void launch_prim_ref(int n, int stride, const double* U, double* V, float* V32, Launch l);
 
-// fast FP64 and mixed FP32/FP64 (kernels_fast.cu)
-// dt, when not null, makes the gradient kernel compute the next step's time
-// step too (the last stage)
-void launch_gradient_fast(const MeshView<double>& m, const StageArgs& a, const DtFuse* dt, Launch l);
-void launch_flux_fast(const MeshView<double>& m, const StageArgs& a, Launch l);
-void launch_gradient_mixed(const MeshView<float>& m, const StageArgs& a, Launch l);
-void launch_flux_mixed(const MeshView<float>& m, const StageArgs& a, Launch l);
-void launch_ghost_fast(const MeshView<double>& m, const StageArgs& a, Launch l);
-void launch_bflux_fast(const MeshView<double>& m, const StageArgs& a, Launch l);
-// mixed: ghosts come from launch_ghost_fast (FP64); boundary fluxes are
-// stored as FP32 differences to the owner's physical flux
-void launch_bflux_mixed(const MeshView<double>& m, const StageArgs& a, Launch l);
+// fast forms (kernels_fast.cu): the stage kernel (kernels_tile.cuh) of a form
+// (kFormFp64, kFormDelta, kFormCopy) over the tiles of a mesh
+struct Tiles;
+struct TileView;
+size_t stage_smem(int form, const Tiles& t, bool second);  // shared memory of a block; 0: the tiles' lists are too long
+// once per device before a launch of a mode (kModeFirst ...); *blocks: blocks a multiprocessor holds
+cudaError_t stage_setup(int form, int tile, int mode, int max_smem, size_t smem, int* blocks);
+void launch_stage(int form, int tile, int mode, const MeshView<double>& m, const TileView& tv, const StageArgs& a,
+                  size_t smem, cudaStream_t st);
+// the form with FP32 copies under the Barth limiter (kernels_copy.cuh)
+void launch_gradient_copy(const MeshView<float>& m, const StageArgs& a, Launch l, int variant);
+void launch_flux_copy(const MeshView<float>& m, const StageArgs& a, Launch l, int variant);
+void launch_bflux_copy(const MeshView<double>& m, const TileView& tv, const StageArgs& a, Launch l);
+// the gradient field of a stage's input (keep_stage_fields)
+void launch_gradient_field(int form, const MeshView<double>& m, const MeshView<float>& m32, const StageArgs& a,
+                           cudaStream_t st);
+// cell-centre ghost states of the stage's input, FP64 or (FP32 copies) FP32
+void launch_ghost(int form, const MeshView<double>& m, const TileView& tv, const StageArgs& a, Launch l);
 void launch_prim_fast(int n, int stride, const double* U, double* V, float* V32, Launch l);
-// mixed with FP32 copies: the FP32 node kernels and the boundary kernels that
-// read and write the FP32 copies (kernels_fast.cu)
-void launch_gradient_m32(const MeshView<float>& m, const StageArgs& a, Launch l);
-void launch_flux_m32(const MeshView<float>& m, const StageArgs& a, Launch l);
-void launch_ghost_m32(const MeshView<double>& m, const StageArgs& a, Launch l);
-void launch_bflux_m32(const MeshView<double>& m, const StageArgs& a, Launch l);
 // the fast forms' reciprocal and reciprocal square root, elementwise (self-test)
 void launch_fastmath(const double* x, int n, double* rcp, double* rsq, Launch l);
 

@@ -534,6 +534,8 @@ Mesh concat_meshes(const std::vector<const Mesh*>& parts) {
   return m;
 }
 
+int build_threads(size_t n) { return host_threads(n); }
+
 }  // namespace nf
 
 extern "C" int nf_set_host_threads(int n) {

@@ -67,6 +67,9 @@ Mesh build_mesh(const std::vector<double>& nodes, const std::vector<int64_t>& te
 // Parse an SU2 file; names/types give every marker's boundary type.
 Mesh read_su2(const std::string& path, const std::vector<std::string>& names, const std::vector<int>& types);
 
+// Host threads a loop over n elements may use (nf_set_host_threads, the environment override).
+int build_threads(size_t n);
+
 Mesh concat_meshes(const std::vector<const Mesh*>& parts);
 
 // The same Mesh, bit for bit, built on the current CUDA device

@@ -4,7 +4,8 @@
 // every device buffer, one stream and the CUDA graphs of the step, and
 // enqueues per step:
 //   [dt reset + timestep kernel]   EulerSolver::calc_timestep
-//   per stage: gradient_limiter, flux_update
+//   per stage: [ghost kernel], then the stage kernel (fast forms) or the
+//              gradient, boundary flux and flux kernels (reference order)
 //   [end-of-step kernel]           time += dt (Driver.cpp:47), validity of dt
 // The primitives of successive stage inputs alternate between two buffers, so
 // the buffer that fed the last stage still holds them when the next
@@ -23,6 +24,7 @@
 
 #include "../../include/netflux_b200.h"
 #include "launch.hpp"
+#include "kernels_tile.cuh"
 #include "mesh.hpp"
 
 
@@ -259,15 +261,24 @@ struct nf_solver {
   std::string err;
 
   // mesh
-  DevBuf<int> slot, nbslot, b_cell, b_slot, b_face, b_patch, b_slotf;
-  DevBuf<int> cnode, gcode, nbvf, nbsf;  // node-based layout of the fast forms
+  DevBuf<int> slot, nbslot, b_cell, b_slot, b_face, b_patch;  // boundary faces of the reference-order form
+  DevBuf<int> cnode, gcode, nbvf, nbsf;  // node-based layout of the fast forms (nbsf: copy_barth)
   DevBuf<double> S, nhat, area, rs, vol, dS, nodes4;
   DevBuf<float> nodes4_32;
+  // tiles of the fast forms' stage kernel
+  DevBuf<nf::TileHead> tile_head;
+  DevBuf<uint16_t> tile_code, tile_vert, cut_nb;
+  DevBuf<int> cut_cell, far_id, tile_node;
+  DevBuf<double4> b_geo;
+  DevBuf<int2> b_ref;
+  int tile = 0, n_tiles = 0, ahead = 0;
+  int stage_mode = 0;  // kModeFirst ... kModeGeneral
+  size_t stage_smem = 0;
   int nb = 0, bstride = 0;
   DevBuf<nf::PatchBC> patches;
   // state
-  DevBuf<double> U, W, V0, V1, fs, grad, phi, R, dt_local, res_cell, scal, part, res_out, vg, fb;
-  // FP64 form: the last stage also computes the next step's dt, into the
+  DevBuf<double> U, W, V0, V1, fs, grad, phi, R, dt_local, res_cell, scal, part, res_out, vg, vgb, fb;
+  // fast forms: a stage also computes the next step's dt (dt_stage), into the
   // other per-cell dt buffer (dtl_cur names the one the next step uses);
   // dt_ready says the next step's dt is already on the device
   DevBuf<double> dt_local2;
@@ -275,11 +286,11 @@ struct nf_solver {
   bool dt_ready = false;
   DevBuf<double> Uold;       // U^n of the next step when set apart from U (nf_set_state_old)
   bool old_pending = false;
-  DevBuf<float> fs32, grad32, phi32, fb32;  // mixed: increments, fields, boundary flux differences
+  DevBuf<float> grad32, phi32;  // mixed: kept stage fields
+  DevBuf<float> fs32, fb32;     // copy_barth: face states, boundary fluxes
   // mixed with FP32 copies: FP32 primitives of successive stage inputs (the
-  // same double-buffering as V0/V1) and FP32 ghost states; fs32 and fb32
-  // hold its face states and boundary fluxes
-  DevBuf<float> V32a, V32b, vg32;
+  // same double-buffering as V0/V1) and FP32 ghost states
+  DevBuf<float> V32a, V32b, vg32, vg32b;
   DevBuf<unsigned> status;
   DevBuf<long long> chunk_begin, chunk_end, case_cells;
   DevBuf<int> case_chunk0;
@@ -308,13 +319,13 @@ struct nf_solver {
   int vcur = 0;              // V buffer holding the primitives of the current state
   bool stepped = false;
   cudaGraphExec_t graph[2] = {nullptr, nullptr};  // two steps from vcur = 0 / 1
-  // launch configuration of the gradient and flux kernels (fast forms)
+  // launch shapes as nf_set_launch_shapes takes and nf_tune reports them; the
+  // stage kernel's shape follows from the mesh
   struct KCfg {
     int block = 128;
     int variant = 0;
   };
   KCfg kgrad, kflux;
-  bool tuned = false;
   DevBuf<double> stage;           // AoS staging for state transfers [N][5]
   // asynchronous state snapshots (nf_snapshot_begin / nf_snapshot_wait): a
   // second AoS staging buffer, copied to the host on its own stream
@@ -366,22 +377,40 @@ struct nf_solver {
     prof_used++;
   }
 
+  // Fast forms, second order: ghost buffer i goes with primitive buffer i. A stage
+  // kernel leaves its result's ghosts; ghosts_ready says those of the current
+  // primitives are in place, and whatever else writes primitives clears it.
+  // Up to kGhostWaves waves of tiles a kernel of its own (4 us a stage, mostly
+  // launch) costs more than the boundary tiles' longer stay, beyond it less:
+  // a step of 48,000 tets 50 -> 46 us, of 393,216 (4 waves) 175 -> 174 us, of
+  // 3.1M (28 waves) 1.161 -> 1.167 ms.
+  static constexpr int kGhostWaves = 6;
+  bool own_ghosts() const { return n_tiles <= kGhostWaves * ahead && !copy_barth(); }  // the stage kernel leaves them
+  bool ghosts_ready = false;
+  double* vgbuf(int i) { return i && fast() ? vgb.p : vg.p; }
+  float* vg32buf(int i) { return i ? vg32b.p : vg32.p; }
+
   double* Vbuf(int i) { return i ? V1.p : V0.p; }
   float* V32buf(int i) { return i ? V32b.p : V32a.p; }
   // the conserved state stage s reads (Solver.cpp:103-133: U, then the RK
   // stage W)
   double* stage_input(int s) { return (p.time_scheme == NF_TVD_RK3 && s > 0) ? W.p : U.p; }
   double* dtl(int i) { return i ? dt_local2.p : dt_local.p; }
-  // the FP64 form's last stage computes the next step's dt (second order:
-  // its gradient kernel reads the primitives the reference's dt reads)
-  bool fuse_dt() const {
-    return p.precision == NF_PREC_FP64 && p.spatial_order == NF_SECOND_ORDER && !p.dt_from_current_state;
+  // the form with FP32 copies under the limiter has its own kernels (kernels_copy.cuh)
+  bool copy_barth() const {
+    return p.precision == NF_PREC_MIXED32 && p.spatial_order == NF_SECOND_ORDER && p.limiter == NF_LIMITER_BARTH;
   }
-  // the mixed forms (TVD-RK3): the stage-2 flux kernel computes the next
-  // step's dt from the primitives of its result, the last stage's input
-  bool fuse_dt_flux() const {
-    return (p.precision == NF_PREC_MIXED || p.precision == NF_PREC_MIXED32) && p.time_scheme == NF_TVD_RK3 &&
-           !p.dt_from_current_state;
+  bool fast() const { return p.precision != NF_PREC_FP64_REF; }
+  int form() const {
+    return p.precision == NF_PREC_FP64 ? nf::kFormFp64 : p.precision == NF_PREC_MIXED ? nf::kFormDelta : nf::kFormCopy;
+  }
+  // the stage that computes the next step's dt in the fast forms (StageArgs::
+  // dt_from_input): the last one from its input, or with FP32 copies stage 2 of 3
+  // from its result; -1: none (timestep_kernel does)
+  int dt_stage() const {
+    if (!fast() || p.dt_from_current_state) return -1;
+    if (p.precision != NF_PREC_MIXED32) return n_stages() - 1;
+    return p.time_scheme == NF_TVD_RK3 ? n_stages() - 2 : -1;
   }
   // primitives of Usrc into primitive buffer b (and its FP32 copy in the
   // mixed form with FP32 copies)
@@ -393,17 +422,32 @@ struct nf_solver {
   nf::Launch launch() const { return nf::Launch{block, stream}; }
 
   nf::MeshView<double> view64() const {
-    const bool fast = p.precision != NF_PREC_FP64_REF;
     return nf::MeshView<double>{n, stride, n_faces, slot.p, nbslot.p, S.p, nhat.p, area.p, rs.p,
                                 nodes4.p, cnode.p, gcode.p, nbvf.p, nbsf.p, vol.p, dS.p, patches.p, nb,
-                                bstride, b_cell.p, b_slot.p, b_face.p, b_patch.p, fast ? b_slotf.p : b_slot.p,
+                                bstride, b_cell.p, b_slot.p, b_face.p, b_patch.p,
                                 int(n_nodes), int(patches.n)};
   }
   nf::MeshView<float> view32() const {
     return nf::MeshView<float>{n, stride, n_faces, slot.p, nbslot.p, nullptr, nullptr, nullptr, nullptr,
                                nodes4_32.p, cnode.p, gcode.p, nbvf.p, nbsf.p, vol.p, dS.p, patches.p, nb,
-                               bstride, b_cell.p, b_slot.p, b_face.p, b_patch.p, b_slotf.p, int(n_nodes),
+                               bstride, b_cell.p, b_slot.p, b_face.p, b_patch.p, int(n_nodes),
                                int(patches.n)};
+  }
+
+  nf::TileView tiles() const {
+    return nf::TileView{tile_head.p,
+                        reinterpret_cast<const uint2*>(tile_code.p),
+                        reinterpret_cast<const uint2*>(tile_vert.p),
+                        cut_cell.p,
+                        reinterpret_cast<const ushort4*>(cut_nb.p),
+                        far_id.p,
+                        tile_node.p,
+                        p.precision == NF_PREC_FP64 ? static_cast<const void*>(nodes4.p)
+                                                    : static_cast<const void*>(nodes4_32.p),
+                        b_geo.p,
+                        b_ref.p,
+                        n_tiles,
+                        ahead};
   }
 
   void enqueue_dt() {
@@ -428,6 +472,7 @@ struct nf_solver {
   // primitives of U in both V buffers (as after nf_set_state)
   void refresh_primitives() {
     for (int b = 0; b < 2; b++) launch_prim(U.p, b);
+    ghosts_ready = false;
   }
 
   void ratchet_reset() {
@@ -460,6 +505,11 @@ struct nf_solver {
     return std::min<int64_t>(n, p.limiter_ratchet_step - steps_done);
   }
 
+  // the captured steps take the ghosts as the step before left them
+  bool graph_ready() const {
+    return !fast() || p.spatial_order != NF_SECOND_ORDER || ghosts_ready || !own_ghosts();
+  }
+
   // n x (calc_timestep + step), replays of a two-step CUDA graph where
   // possible; the ratchet starts at its step.
   void run_steps(int64_t n) {
@@ -474,7 +524,7 @@ struct nf_solver {
       int64_t left = ratchet_due(n);
       n -= left;
       steps_done += left;
-      if (left >= 2 && stepped) {
+      if (left >= 2 && stepped && graph_ready()) {
         const int v0 = vcur;
         if (!graph[v0]) {
           // capture two steps: the V buffers return to their roles afterwards
@@ -498,37 +548,19 @@ struct nf_solver {
         enqueue_dt();
         enqueue_step();
         left--;
+        // the rest by graph, where there is one or its capture (about 0.2 ms) pays
+        if (left >= (graph[vcur] ? 2 : 32) && graph_ready()) break;
       }
+      n += left;
+      steps_done -= left;
     }
   }
 
-  void launch_gradient(const nf::StageArgs& a, const KCfg& k, const nf::DtFuse* dtf = nullptr) {
-    const nf::Launch l{k.block, stream, k.variant};
-    if (p.precision == NF_PREC_MIXED) nf::launch_gradient_mixed(view32(), a, l);
-    else if (p.precision == NF_PREC_MIXED32) nf::launch_gradient_m32(view32(), a, l);
-    else if (p.precision == NF_PREC_FP64) nf::launch_gradient_fast(view64(), a, dtf, l);
-    else nf::launch_gradient_ref(view64(), a, launch());
-  }
-  void launch_flux(const nf::StageArgs& a, const KCfg& k) {
-    const nf::Launch l{k.block, stream, k.variant};
-    if (p.precision == NF_PREC_MIXED) nf::launch_flux_mixed(view32(), a, l);
-    else if (p.precision == NF_PREC_MIXED32) nf::launch_flux_m32(view32(), a, l);
-    else if (p.precision == NF_PREC_FP64) nf::launch_flux_fast(view64(), a, l);
-    else nf::launch_flux_ref(view64(), a, launch());
-  }
-  // ghost states and boundary fluxes of the stage, in each form's precision
   void launch_ghost(const nf::StageArgs& a) {
     if (p.precision == NF_PREC_FP64_REF) nf::launch_ghost_ref(view64(), a, launch());
-    else if (p.precision == NF_PREC_MIXED32) nf::launch_ghost_m32(view64(), a, launch());
-    else nf::launch_ghost_fast(view64(), a, launch());
+    else nf::launch_ghost(form(), view64(), tiles(), a, launch());
   }
-  void launch_bflux(const nf::StageArgs& a) {
-    if (p.precision == NF_PREC_MIXED) nf::launch_bflux_mixed(view64(), a, launch());
-    else if (p.precision == NF_PREC_MIXED32) nf::launch_bflux_m32(view64(), a, launch());
-    else if (p.precision == NF_PREC_FP64) nf::launch_bflux_fast(view64(), a, launch());
-    else nf::launch_bflux_ref(view64(), a, launch());
-  }
-  // launch variants the tuner may pick (gradient, flux)
+  // launch variants accepted by nf_set_launch_shapes (gradient, flux)
   int grad_variants() const { return 10; }
   int flux_variants() const { return 10; }
 
@@ -543,15 +575,10 @@ struct nf_solver {
     a.local_dt = p.local_time_stepping;
     a.Vin = Vbuf(vcur);
     a.Vout = Vbuf(1 - vcur);
-    a.fs = fs.p;
-    a.vg = vg.p;
-    a.fb = fb.p;
     a.fb32 = fb32.p;
-    if (p.precision == NF_PREC_MIXED32) {
-      a.Vin32 = V32buf(vcur);
-      a.Vout32 = V32buf(1 - vcur);
-      a.vg32 = vg32.p;
-    }
+    a.Vin32 = V32buf(vcur);
+    a.Vout32 = V32buf(1 - vcur);
+    a.vg32 = vg32buf(vcur);
     a.dt_local = dtl(dtl_cur);
     a.scal = scal.p;
     a.status = status.p;
@@ -564,17 +591,14 @@ struct nf_solver {
   // Pick block size and variant of the gradient and flux kernels by timing
   // each candidate on the current state (CUDA events on this stream).
   void tune() {
-    tuned = true;
-    if (p.precision == NF_PREC_FP64_REF) return;  // reference form: fixed shape
+    if (!copy_barth()) return;  // the other forms' shapes are fixed
     const int other = 1 - vcur;
     std::vector<double> keep(size_t(5) * stride);
-    std::vector<float> keep32(p.precision == NF_PREC_MIXED32 ? size_t(5) * stride : 0);
+    std::vector<float> keep32(size_t(5) * stride);
     ck(cudaMemcpyAsync(keep.data(), Vbuf(other), keep.size() * sizeof(double), cudaMemcpyDeviceToHost, stream),
        "tune save");
-    if (!keep32.empty())
-      ck(cudaMemcpyAsync(keep32.data(), V32buf(other), keep32.size() * sizeof(float), cudaMemcpyDeviceToHost,
-                         stream),
-         "tune save");
+    ck(cudaMemcpyAsync(keep32.data(), V32buf(other), keep32.size() * sizeof(float), cudaMemcpyDeviceToHost, stream),
+       "tune save");
     ck(cudaStreamSynchronize(stream), "tune sync");
     nf::StageArgs a = first_stage_args();
     cudaEvent_t e0, e1;
@@ -596,35 +620,27 @@ struct nf_solver {
         for (int v = 0; v < n_variants; v++) c.push_back(KCfg{b, v});
       return c;
     };
-    if (a.second_order) {
-      launch_ghost(a);
+    const nf::MeshView<float> m = view32();
+    auto best_of = [&](int n_variants, KCfg& keep_cfg, auto&& fn) {
       float best = 1e30f;
-      for (const KCfg& k : cands(grad_variants())) {
-        const float t = time_it([&] { launch_gradient(a, k); });
+      for (const KCfg& k : cands(n_variants)) {
+        const float t = time_it([&] { fn(nf::Launch{k.block, stream}, k.variant); });
         if (t < best) {
           best = t;
-          kgrad = k;
+          keep_cfg = k;
         }
       }
-      launch_gradient(a, kgrad);
-    }
-    launch_bflux(a);
-    float best = 1e30f;
-    for (const KCfg& k : cands(flux_variants())) {
-      const float t = time_it([&] { launch_flux(a, k); });
-      if (t < best) {
-        best = t;
-        kflux = k;
-      }
-    }
+    };
+    launch_ghost(a);
+    best_of(grad_variants(), kgrad, [&](nf::Launch l, int v) { nf::launch_gradient_copy(m, a, l, v); });
+    nf::launch_bflux_copy(view64(), tiles(), a, launch());
+    best_of(flux_variants(), kflux, [&](nf::Launch l, int v) { nf::launch_flux_copy(m, a, l, v); });
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     ck(cudaMemcpyAsync(Vbuf(other), keep.data(), keep.size() * sizeof(double), cudaMemcpyHostToDevice, stream),
        "tune restore");
-    if (!keep32.empty())
-      ck(cudaMemcpyAsync(V32buf(other), keep32.data(), keep32.size() * sizeof(float), cudaMemcpyHostToDevice,
-                         stream),
-         "tune restore");
+    ck(cudaMemcpyAsync(V32buf(other), keep32.data(), keep32.size() * sizeof(float), cudaMemcpyHostToDevice, stream),
+       "tune restore");
     ck(cudaMemsetAsync(status.p, 0, sizeof(unsigned), stream), "status reset");
     ck(cudaStreamSynchronize(stream), "tune sync");
     for (auto& g : graph)
@@ -645,9 +661,7 @@ struct nf_solver {
   // One stage of the step; the last one also ends the step.
   void enqueue_stage(int s) {
     const int n_stages = this->n_stages();
-    const bool fuse = fuse_dt() || fuse_dt_flux();
-    nf::DtFuse dtf{p.cfl, p.local_time_stepping ? dtl(1 - dtl_cur) : nullptr,
-                   reinterpret_cast<unsigned long long*>(scal.p + nf::kScalDtNext)};
+    const bool fuse = dt_stage() >= 0;
     {
       nf::StageArgs a{};
       a.second_order = p.spatial_order == NF_SECOND_ORDER;
@@ -661,9 +675,8 @@ struct nf_solver {
       a.Vin = Vbuf(vcur);
       a.Vout = Vbuf(1 - vcur);
       a.fs = fs.p;
-      a.vg = vg.p;
+      a.vg = vgbuf(vcur);
       a.fb = fb.p;
-      a.fb32 = fb32.p;
       a.grad = p.keep_stage_fields ? grad.p : nullptr;
       a.phi = p.keep_stage_fields ? phi.p : nullptr;
       a.R = p.keep_stage_fields ? R.p : nullptr;
@@ -694,39 +707,72 @@ struct nf_solver {
       if (p.precision == NF_PREC_MIXED32) {
         a.Vin32 = V32buf(vcur);
         a.Vout32 = V32buf(1 - vcur);
-        a.vg32 = vg32.p;
+        a.vg32 = vg32buf(vcur);
         // the FP64 primitives only where a time-step kernel reads them: the
         // state the next time step reads (the last stage's input, Q3, or with
         // dt_from_current_state the step's result), unless the stage-2 flux
         // kernel computes that time step itself from its FP64 result
-        const int dt_stage = p.dt_from_current_state ? n_stages - 1 : std::max(n_stages - 2, 0);
-        if (s != dt_stage || fuse_dt_flux()) a.Vout = nullptr;
+        const int read_stage = p.dt_from_current_state ? n_stages - 1 : std::max(n_stages - 2, 0);
+        if (s != read_stage || fuse) a.Vout = nullptr;
       }
-      if (fuse_dt_flux() && s == n_stages - 2) {
-        a.dt_next = dtf.dt_next;
-        a.dt_next_min = dtf.dt_min_bits;
+      if (fuse && s == dt_stage()) {
+        a.dt_from_input = p.precision != NF_PREC_MIXED32;
+        a.dt_next = p.local_time_stepping ? dtl(1 - dtl_cur) : nullptr;
+        a.dt_next_min = reinterpret_cast<unsigned long long*>(scal.p + nf::kScalDtNext);
         a.dS = dS.p;
         a.cfl = p.cfl;
       }
       if (p.precision == NF_PREC_MIXED || p.precision == NF_PREC_MIXED32) {
-        a.fs32 = fs32.p;
         a.grad32 = p.keep_stage_fields ? grad32.p : nullptr;
         a.phi32 = p.keep_stage_fields ? phi32.p : nullptr;
       }
-      if (a.second_order) {
+      if (a.second_order && !(fast() && ghosts_ready)) {
         prof_begin(NF_KERNEL_OTHER);
         launch_ghost(a);
         prof_end();
-        prof_begin(NF_KERNEL_GRADIENT);
-        launch_gradient(a, kgrad, (fuse_dt() && s == n_stages - 1) ? &dtf : nullptr);
+      }
+      ghosts_ready = false;
+      if (fast() && a.second_order && own_ghosts()) {
+        if (p.precision == NF_PREC_MIXED32) a.vg_next32 = vg32buf(1 - vcur);
+        else a.vg_next = vgbuf(1 - vcur);
+        ghosts_ready = true;
+      }
+      if (fast()) {
+        if (a.second_order && p.keep_stage_fields) {
+          prof_begin(NF_KERNEL_GRADIENT);
+          nf::launch_gradient_field(form(), view64(), view32(), a, stream);
+          prof_end();
+        }
+        if (copy_barth()) {
+          a.fs32 = fs32.p;
+          a.fb32 = fb32.p;
+          prof_begin(NF_KERNEL_GRADIENT);
+          nf::launch_gradient_copy(view32(), a, nf::Launch{kgrad.block, stream}, kgrad.variant);
+          prof_end();
+          prof_begin(NF_KERNEL_OTHER);
+          nf::launch_bflux_copy(view64(), tiles(), a, launch());
+          prof_end();
+          prof_begin(NF_KERNEL_FLUX);
+          nf::launch_flux_copy(view32(), a, nf::Launch{kflux.block, stream}, kflux.variant);
+          prof_end();
+        } else {
+          prof_begin(NF_KERNEL_FLUX);
+          nf::launch_stage(form(), tile, stage_mode, view64(), tiles(), a, stage_smem, stream);
+          prof_end();
+        }
+      } else {
+        if (a.second_order) {
+          prof_begin(NF_KERNEL_GRADIENT);
+          nf::launch_gradient_ref(view64(), a, launch());
+          prof_end();
+        }
+        prof_begin(NF_KERNEL_OTHER);
+        nf::launch_bflux_ref(view64(), a, launch());
+        prof_end();
+        prof_begin(NF_KERNEL_FLUX);
+        nf::launch_flux_ref(view64(), a, launch());
         prof_end();
       }
-      prof_begin(NF_KERNEL_OTHER);
-      launch_bflux(a);
-      prof_end();
-      prof_begin(NF_KERNEL_FLUX);
-      launch_flux(a, kflux);
-      prof_end();
       vcur = 1 - vcur;
     }
     if (s < n_stages - 1) return;
@@ -773,6 +819,7 @@ struct nf_solver {
     const int st = stride;
     scatter_state_kernel<<<(n + 255) / 256, 256, 0, stream>>>(n, st, d_dev_of_ref.p, aos, U.p);
     for (int b = 0; b < 2; b++) launch_prim(U.p, b);
+    ghosts_ready = false;
     vcur = 0;
     dtl_cur = 0;
     dt_ready = false;
@@ -867,6 +914,7 @@ struct nf_split {
       halo_copy_kernel<<<int((lk->n + 255) / 256), 256, 0, b->stream>>>(
           lk->n, a->stride, lk->from_cells.p, a->Vbuf(a->vcur), a->stage_input(k), b->stride, lk->to_cells.p,
           b->Vbuf(b->vcur), b->stage_input(k));
+      b->ghosts_ready = false;  // halo cells may have boundary faces
       ck(cudaGetLastError(), "halo copy launch");
     }
     for (size_t i = 0; i < parts.size(); i++) {
@@ -1117,7 +1165,6 @@ nf_solver* nf_create(const nf_mesh* h, const nf_params* params) {
       s->kgrad.block = s->kflux.block = std::min(p.block_size, 128);
       s->kgrad.variant = std::max(0, std::min(p.kernel_variant, s->grad_variants() - 1));
       s->kflux.variant = std::max(0, std::min(p.kernel_variant, s->flux_variants() - 1));
-      s->tuned = true;  // a caller-fixed shape is not tuned
     }
     if (s->block % 32 || s->block > 256) throw std::runtime_error("block_size must be a multiple of 32, <= 256");
     if (p.device >= 0) ck(cudaSetDevice(p.device), "cudaSetDevice");
@@ -1136,74 +1183,99 @@ nf_solver* nf_create(const nf_mesh* h, const nf_params* params) {
     s->n_cases = m.n_cases();
     const int stride = s->stride;
 
-    // device face order: by the first device cell that touches the face
-    std::vector<int64_t> key(static_cast<size_t>(F));
-    for (int64_t f = 0; f < F; f++) {
-      const int64_t di = m.dev_of_ref[m.face_i[size_t(f)]];
-      const bool interior = m.face_j[size_t(f)] < uint32_t(N);
-      key[size_t(f)] = interior ? std::min(di, m.dev_of_ref[m.face_j[size_t(f)]]) : di;
-    }
-    std::vector<int64_t> dev_face_order(static_cast<size_t>(F));
-    std::iota(dev_face_order.begin(), dev_face_order.end(), 0);
-    std::stable_sort(dev_face_order.begin(), dev_face_order.end(),
-                     [&](int64_t a, int64_t b) { return key[size_t(a)] < key[size_t(b)]; });
-    std::vector<int64_t> fdev(static_cast<size_t>(F));
-    for (int64_t k = 0; k < F; k++) fdev[size_t(dev_face_order[size_t(k)])] = k;
-
-    std::vector<double> h_S(size_t(3 * F)), h_n(size_t(3 * F)), h_a(static_cast<size_t>(F));
-    for (int64_t f = 0; f < F; f++) {
-      const int64_t d = fdev[size_t(f)];
-      h_a[size_t(d)] = m.area[size_t(f)];
-      for (int c = 0; c < 3; c++) {
-        h_S[size_t(c * F + d)] = m.S[size_t(3 * f + c)];
-        h_n[size_t(c * F + d)] = m.nhat[size_t(3 * f + c)];
-      }
-    }
-    // slots in reference face order; nbslot names the other side of each face
-    std::vector<int> h_slot(size_t(4) * stride, -1), h_nb(size_t(4) * stride, 0);
-    std::vector<double> h_rs(size_t(12) * stride, 0.0);  // [d][q][cell]
+    const bool fast = p.precision != NF_PREC_FP64_REF;
+    // boundary faces in owner-cell order
     struct BFace {
-      int64_t cell;
-      int q, face, patch;
+      int64_t cell, face;  // device cell, reference face
+      int slot, patch;
     };
     std::vector<BFace> bfaces;
-    std::vector<int> fill(static_cast<size_t>(stride), 0);
-    auto add_slot = [&](int64_t cell_dev, int value) {
-      int& k = fill[size_t(cell_dev)];
-      if (k >= 4) throw std::runtime_error("a cell has more than 4 faces (only tetrahedra are supported)");
-      h_slot[size_t(k) * stride + size_t(cell_dev)] = value;
-      return k++;
-    };
-    for (int64_t f = 0; f < F; f++) {
-      const int fd = int(fdev[size_t(f)]);
-      const int64_t di = m.dev_of_ref[m.face_i[size_t(f)]];
-      const int qi = add_slot(di, fd << 1);
-      for (int c = 0; c < 3; c++) h_rs[(size_t(c) * 4 + qi) * stride + size_t(di)] = m.ri[size_t(3 * f + c)];
-      const uint32_t j = m.face_j[size_t(f)];
-      if (j < uint32_t(N)) {
-        const int64_t dj = m.dev_of_ref[j];
-        const int qj = add_slot(dj, (fd << 1) | 1);
-        for (int c = 0; c < 3; c++) h_rs[(size_t(c) * 4 + qj) * stride + size_t(dj)] = m.rj[size_t(3 * f + c)];
-        h_nb[size_t(qi) * stride + size_t(di)] = int(dj << 2) | qj;
-        h_nb[size_t(qj) * stride + size_t(dj)] = int(di << 2) | qi;
-      } else {
-        bfaces.push_back({di, qi, fd, int(m.face_patch[size_t(f)])});
-      }
-    }
-    // boundary faces in owner-cell order; the owner's slot names its index
+    for (int64_t f = 0; f < F; f++)
+      if (m.face_j[size_t(f)] >= uint32_t(N))
+        bfaces.push_back({m.dev_of_ref[m.face_i[size_t(f)]], f, 0, int(m.face_patch[size_t(f)])});
     std::stable_sort(bfaces.begin(), bfaces.end(), [](const BFace& x, const BFace& y) { return x.cell < y.cell; });
     const int nbf = int(bfaces.size());
-    std::vector<int> hb_cell(static_cast<size_t>(nbf)), hb_slot(static_cast<size_t>(nbf)), hb_face(static_cast<size_t>(nbf)), hb_patch(static_cast<size_t>(nbf));
+    std::vector<int> bindex(static_cast<size_t>(F), -1);  // boundary index of a reference face
+    std::vector<int> hb_cell(static_cast<size_t>(nbf));
     for (int b = 0; b < nbf; b++) {
+      bindex[size_t(bfaces[size_t(b)].face)] = b;
       hb_cell[size_t(b)] = int(bfaces[size_t(b)].cell);
-      hb_slot[size_t(b)] = bfaces[size_t(b)].q;
-      hb_face[size_t(b)] = bfaces[size_t(b)].face;
-      hb_patch[size_t(b)] = bfaces[size_t(b)].patch;
-      h_nb[size_t(bfaces[size_t(b)].q) * stride + size_t(bfaces[size_t(b)].cell)] = -(1 + b);
+    }
+    if (!fast) {
+      // reference-order form. Device face order: by the first device cell that
+      // touches the face
+      std::vector<int64_t> key(static_cast<size_t>(F));
+      for (int64_t f = 0; f < F; f++) {
+        const int64_t di = m.dev_of_ref[m.face_i[size_t(f)]];
+        const bool interior = m.face_j[size_t(f)] < uint32_t(N);
+        key[size_t(f)] = interior ? std::min(di, m.dev_of_ref[m.face_j[size_t(f)]]) : di;
+      }
+      std::vector<int64_t> dev_face_order(static_cast<size_t>(F));
+      std::iota(dev_face_order.begin(), dev_face_order.end(), 0);
+      std::stable_sort(dev_face_order.begin(), dev_face_order.end(),
+                       [&](int64_t a, int64_t b) { return key[size_t(a)] < key[size_t(b)]; });
+      std::vector<int64_t> fdev(static_cast<size_t>(F));
+      for (int64_t k = 0; k < F; k++) fdev[size_t(dev_face_order[size_t(k)])] = k;
+
+      std::vector<double> h_S(size_t(3 * F)), h_n(size_t(3 * F)), h_a(static_cast<size_t>(F));
+      for (int64_t f = 0; f < F; f++) {
+        const int64_t d = fdev[size_t(f)];
+        h_a[size_t(d)] = m.area[size_t(f)];
+        for (int c = 0; c < 3; c++) {
+          h_S[size_t(c * F + d)] = m.S[size_t(3 * f + c)];
+          h_n[size_t(c * F + d)] = m.nhat[size_t(3 * f + c)];
+        }
+      }
+      // slots in reference face order; nbslot names the other side of each face
+      std::vector<int> h_slot(size_t(4) * stride, -1), h_nb(size_t(4) * stride, 0);
+      std::vector<double> h_rs(size_t(12) * stride, 0.0);  // [d][q][cell]
+      std::vector<int> fill(static_cast<size_t>(stride), 0);
+      auto add_slot = [&](int64_t cell_dev, int value) {
+        int& k = fill[size_t(cell_dev)];
+        if (k >= 4) throw std::runtime_error("a cell has more than 4 faces (only tetrahedra are supported)");
+        h_slot[size_t(k) * stride + size_t(cell_dev)] = value;
+        return k++;
+      };
+      for (int64_t f = 0; f < F; f++) {
+        const int fd = int(fdev[size_t(f)]);
+        const int64_t di = m.dev_of_ref[m.face_i[size_t(f)]];
+        const int qi = add_slot(di, fd << 1);
+        for (int c = 0; c < 3; c++) h_rs[(size_t(c) * 4 + qi) * stride + size_t(di)] = m.ri[size_t(3 * f + c)];
+        const uint32_t j = m.face_j[size_t(f)];
+        if (j < uint32_t(N)) {
+          const int64_t dj = m.dev_of_ref[j];
+          const int qj = add_slot(dj, (fd << 1) | 1);
+          for (int c = 0; c < 3; c++) h_rs[(size_t(c) * 4 + qj) * stride + size_t(dj)] = m.rj[size_t(3 * f + c)];
+          h_nb[size_t(qi) * stride + size_t(di)] = int(dj << 2) | qj;
+          h_nb[size_t(qj) * stride + size_t(dj)] = int(di << 2) | qi;
+        } else {
+          const int b = bindex[size_t(f)];
+          bfaces[size_t(b)].slot = qi;
+          h_nb[size_t(qi) * stride + size_t(di)] = -(1 + b);
+        }
+      }
+      // the owner's slot of each boundary face, its face and patch
+      std::vector<int> hb_slot(static_cast<size_t>(nbf)), hb_face(static_cast<size_t>(nbf)),
+          hb_patch(static_cast<size_t>(nbf));
+      for (int b = 0; b < nbf; b++) {
+        hb_slot[size_t(b)] = bfaces[size_t(b)].slot;
+        hb_face[size_t(b)] = int(fdev[size_t(bfaces[size_t(b)].face)]);
+        hb_patch[size_t(b)] = bfaces[size_t(b)].patch;
+      }
+      s->slot.upload(h_slot, st);
+      s->nbslot.upload(h_nb, st);
+      s->rs.upload(h_rs, st);
+      s->S.upload(h_S, st);
+      s->nhat.upload(h_n, st);
+      s->area.upload(h_a, st);
+      s->b_cell.upload(hb_cell, st);
+      s->b_slot.upload(hb_slot, st);
+      s->b_face.upload(hb_face, st);
+      s->b_patch.upload(hb_patch, st);
+      ck(cudaStreamSynchronize(st), "cudaStreamSynchronize");  // the host arrays end here
     }
     // node-based layout of the fast forms: a cell's vertices sorted by node
     // id; face m is the face opposite vertex m
-    const bool fast = p.precision != NF_PREC_FP64_REF;
     std::vector<int> h_cnode, h_gcode, h_nbvf, h_nbsf, hb_slotf;
     if (fast) {
       h_cnode.assign(size_t(4) * stride, 0);
@@ -1254,8 +1326,6 @@ nf_solver* nf_create(const nf_mesh* h, const nf_params* params) {
         *inward = dd < 0.0;
       };
       hb_slotf.assign(size_t(nbf), 0);
-      std::vector<int> bindex(static_cast<size_t>(F), -1);  // boundary index of a device face
-      for (int b = 0; b < nbf; b++) bindex[size_t(bfaces[size_t(b)].face)] = b;
       for (int64_t f = 0; f < F; f++) {
         const int64_t ci = m.face_i[size_t(f)];
         const int64_t di = m.dev_of_ref[size_t(ci)];
@@ -1276,7 +1346,7 @@ nf_solver* nf_create(const nf_mesh* h, const nf_params* params) {
           h_nbsf[size_t(mi) * stride + size_t(di)] = int(dj << 2) | mj;
           h_nbsf[size_t(mj) * stride + size_t(dj)] = int(di << 2) | mi;
         } else {
-          const int b = bindex[size_t(fdev[size_t(f)])];
+          const int b = bindex[size_t(f)];
           h_nbvf[size_t(mi) * stride + size_t(di)] = -(1 + b);
           h_nbsf[size_t(mi) * stride + size_t(di)] = -(1 + b);
           hb_slotf[size_t(b)] = mi;
@@ -1307,19 +1377,60 @@ nf_solver* nf_create(const nf_mesh* h, const nf_params* params) {
       if (b.type < 0 || b.type > 2) throw std::runtime_error("bad boundary type");
     }
 
-    s->slot.upload(h_slot, st);
-    s->nbslot.upload(h_nb, st);
-    s->b_cell.upload(hb_cell, st);
-    s->b_slot.upload(hb_slot, st);
-    s->b_face.upload(hb_face, st);
-    s->b_patch.upload(hb_patch, st);
-    s->rs.upload(h_rs, st);
     if (fast) {
       s->gcode.upload(h_gcode, st);
-      s->b_slotf.upload(hb_slotf, st);
       s->cnode.upload(h_cnode, st);
       s->nbvf.upload(h_nbvf, st);
-      s->nbsf.upload(h_nbsf, st);
+      if (!s->copy_barth()) {
+        int max_smem = 0;
+        ck(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device), "attr");
+        const bool second = p.spatial_order == NF_SECOND_ORDER;
+        nf::Tiles tl;
+        for (int tile : {256, 128, 64}) {
+          tl = nf::build_tiles(s->n, stride, tile, h_nbvf, h_nbsf, h_cnode, h_gcode, hb_cell);
+          const size_t b = nf::stage_smem(s->form(), tl, second);
+          if (b > 0 && b <= size_t(max_smem)) break;
+        }
+        bool open = false;  // some face is not listed
+        for (int ti = 0, cs = 0; ti < tl.n_tiles; ti++) {
+          const int64_t c0 = int64_t(ti) * tl.tile, c1 = std::min(N, c0 + tl.tile);
+          while (m.case_offsets[size_t(cs) + 1] <= c0) cs++;
+          open = open || tl.head[size_t(ti)].open;
+          tl.head[size_t(ti)].case_id = m.case_offsets[size_t(cs) + 1] >= c1 ? cs : -1;
+        }
+        s->tile = tl.tile;
+        s->n_tiles = tl.n_tiles;
+        s->stage_smem = nf::stage_smem(s->form(), tl, second);
+        int per_sm = 0, n_sm = 0;
+        ck(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, s->device), "attr");
+        const bool ratchets = p.limiter == NF_LIMITER_BARTH && (p.limiter_ratchet_step > 0 || p.limiter_ratchet_drop > 0.0);
+        auto setup = [&](int mode) {
+          s->stage_mode = mode;
+          ck(nf::stage_setup(s->form(), s->tile, mode, max_smem, s->stage_smem, &per_sm), "stage kernel set-up");
+          s->ahead = std::max(1, per_sm) * n_sm;
+        };
+        if (!second) setup(nf::kModeFirst);
+        else if (open || ratchets || p.keep_stage_fields) setup(nf::kModeGeneral);
+        else setup(nf::kModePlain);
+        if (s->stage_mode == nf::kModePlain && s->own_ghosts()) setup(nf::kModeGhosts);
+        s->tile_head.upload(tl.head, st);
+        s->tile_code.upload(tl.code, st);
+        s->tile_vert.upload(tl.vert, st);
+        s->cut_cell.upload(tl.cut_cell, st);
+        s->cut_nb.upload(tl.cut_nb, st);
+        s->far_id.upload(tl.far_id, st);
+        s->tile_node.upload(tl.node_id, st);
+      }
+      std::vector<double4> h_bgeo(static_cast<size_t>(nbf));
+      std::vector<int2> h_bref(static_cast<size_t>(nbf));
+      for (int b = 0; b < nbf; b++) {
+        const int64_t f = bfaces[size_t(b)].face;
+        h_bgeo[size_t(b)] = double4{m.nhat[size_t(3 * f)], m.nhat[size_t(3 * f + 1)], m.nhat[size_t(3 * f + 2)],
+                                    m.area[size_t(f)]};
+        h_bref[size_t(b)] = int2{hb_cell[size_t(b)] << 2 | hb_slotf[size_t(b)], bfaces[size_t(b)].patch};
+      }
+      s->b_geo.upload(h_bgeo, st);
+      s->b_ref.upload(h_bref, st);
       std::vector<double> n4(size_t(4) * m.n_nodes, 0.0);
       for (int64_t v = 0; v < m.n_nodes; v++)
         for (int e = 0; e < 3; e++) n4[size_t(4 * v + e)] = m.nodes[size_t(3 * v + e)];
@@ -1330,24 +1441,26 @@ nf_solver* nf_create(const nf_mesh* h, const nf_params* params) {
         s->nodes4_32.upload(n4f, st);
       }
     }
-    s->S.upload(h_S, st);
-    s->nhat.upload(h_n, st);
-    s->area.upload(h_a, st);
     s->vol.upload(h_vol, st);
     s->dS.upload(h_dS, st);
     s->patches.upload(h_pb, st);
     const bool fp32_fields = p.precision == NF_PREC_MIXED || p.precision == NF_PREC_MIXED32;
+    if (s->copy_barth()) {
+      s->fs32.alloc(size_t(20) * stride);
+      s->fs32.zero(st);
+      s->fb32.alloc(size_t(5) * s->bstride);
+      s->fb32.zero(st);
+      s->nbsf.upload(h_nbsf, st);
+    }
     if (p.precision == NF_PREC_MIXED32) {
       s->V32a.alloc(size_t(5) * stride);
       s->V32b.alloc(size_t(5) * stride);
       s->vg32.alloc(size_t(5) * s->bstride);
       s->vg32.zero(st);
+      s->vg32b.alloc(size_t(5) * s->bstride);
+      s->vg32b.zero(st);
     }
     if (fp32_fields) {
-      s->fb32.alloc(size_t(5) * s->bstride);
-      s->fb32.zero(st);
-      s->fs32.alloc(size_t(20) * stride);
-      s->fs32.zero(st);
       if (p.keep_stage_fields) {
         s->grad32.alloc(size_t(15) * stride);
         s->phi32.alloc(size_t(5) * stride);
@@ -1361,7 +1474,11 @@ nf_solver* nf_create(const nf_mesh* h, const nf_params* params) {
     s->V1.alloc(size_t(5) * stride);
     s->vg.alloc(size_t(5) * s->bstride);  // FP64 ghosts in every form
     s->vg.zero(st);
-    if (!fp32_fields) {
+    if (fast) {
+      s->vgb.alloc(size_t(5) * s->bstride);
+      s->vgb.zero(st);
+    }
+    if (!fast) {
       s->fs.alloc(size_t(20) * stride);
       s->fs.zero(st);
       s->fb.alloc(size_t(5) * s->bstride);
@@ -1695,6 +1812,7 @@ int nf_halo_unpack(nf_solver* s, const int64_t* cells, int64_t n, const double* 
     if (rc != NF_OK || n == 0) return rc;
     halo_unpack_kernel<<<int((n + 255) / 256), 256, 0, s->stream>>>(n, s->stride, cells, buf, s->Vbuf(s->vcur),
                                                                      s->stage_input(s->stage_next));
+    s->ghosts_ready = false;
     ck(cudaGetLastError(), "halo unpack");
     ck(cudaStreamSynchronize(s->stream), "cudaStreamSynchronize");
     return NF_OK;
@@ -1938,7 +2056,7 @@ int nf_time_steps(nf_solver* s, int64_t n_steps, int per_kernel, double* ms_tota
     }
     ck(cudaEventRecord(e0, s->stream), "cudaEventRecord");
     int64_t left = n_steps;
-    if (!per_kernel && left >= 2 && s->stepped) {
+    if (!per_kernel && left >= 2 && s->stepped && s->graph_ready()) {
       const int v0 = s->vcur;
       if (!s->graph[v0]) {
         cudaGraph_t g = nullptr;
@@ -2023,7 +2141,6 @@ int nf_set_launch_shapes(nf_solver* s, const int* config) {
     s->kgrad.variant = config[1];
     s->kflux.block = config[2];
     s->kflux.variant = config[3];
-    s->tuned = true;
     for (auto& g : s->graph)
       if (g) {
         cudaGraphExecDestroy(g);

@@ -34,7 +34,7 @@ LIMITERS = {"NONE": L.NF_LIMITER_NONE, "Barth": L.NF_LIMITER_BARTH}
 PRECISIONS = {"fp64_ref": L.NF_PREC_FP64_REF, "fp64": L.NF_PREC_FP64, "mixed": L.NF_PREC_MIXED,
               "mixed32": L.NF_PREC_MIXED32}
 STANDARD_AIR = (1.225, 0.0, 0.0, 0.0, 101325.0)  # Utilities.hpp:100-107
-# launch variants of the gradient and flux kernels each arithmetic form offers (the tuner's candidates)
+# launch variants (gradient, flux) set_launch_shapes accepts for each arithmetic form
 LAUNCH_VARIANTS = {"fp64_ref": (10, 10), "fp64": (10, 10), "mixed": (10, 10), "mixed32": (10, 10)}
 
 
@@ -330,13 +330,13 @@ class EulerSolver:
         return t.value
 
     def tune(self):
-        """Time the gradient/flux launch shapes on the current state and keep the fastest."""
+        """Time the launch shapes where there is a choice and keep the fastest (see nf_tune)."""
         cfg = (C.c_int * 4)()
         _check(L.load().nf_tune(self._h, cfg), self._h)
         return {"gradient": {"block": cfg[0], "variant": cfg[1]}, "flux": {"block": cfg[2], "variant": cfg[3]}}
 
     def set_launch_shapes(self, gradient=(64, 0), flux=(64, 0)):
-        """Fix the gradient/flux launch shapes, each (block, variant) as tune() reports them."""
+        """Set the shapes tune() reports, each (block, variant); see nf_set_launch_shapes."""
         cfg = (C.c_int * 4)(int(gradient[0]), int(gradient[1]), int(flux[0]), int(flux[1]))
         _check(L.load().nf_set_launch_shapes(self._h, cfg), self._h)
 

@@ -53,6 +53,64 @@ def test_one_step_against_reference_order(n, listed, precision, tol):
         assert rel_linf(out[precision], out["fp64_ref"]) <= tol, kw
 
 
+def _shuffled(n_hex, n_bits_lost):
+    """A box of n_hex^3 hexes whose cells come in random order and share one key of the renumbering
+    (a far hex stretches the bounding box), so tiles hold cells from all over the mesh."""
+    m = mg.box_tet_mesh(n_hex, n_hex, n_hex, jitter=0.1, seed=5)
+    far = mg.box_tet_mesh(1, 1, 1, lo=(2.0 ** n_bits_lost,) * 3, hi=(2.0 ** n_bits_lost * 1.5,) * 3)
+    rng = np.random.default_rng(11)
+    tets = np.concatenate([m.tets, far.tets + m.nodes.shape[0]])
+    tris = np.concatenate([m.markers[0][1], far.markers[0][1] + m.nodes.shape[0]])
+    return mg.TetMesh(np.concatenate([m.nodes, far.nodes]), tets[rng.permutation(tets.shape[0])],
+                      [("farfield", tris)], {"farfield": mg.FAR_FIELD})
+
+
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-12), ("mixed", 1e-5), ("mixed32", 1e-5)])
+@pytest.mark.parametrize("n_hex", [3, 7])
+def test_badly_ordered_mesh(n_hex, precision, tol):
+    """Cells without locality: most faces leave their tile, whose lists are the longest they can be
+    (the smallest tile size takes them)."""
+    m = _shuffled(n_hex, 24)
+    U0 = _state(m)
+    mesh = S.Mesh.from_tet_mesh(m)
+    out = {}
+    for prec in ("fp64_ref", precision):
+        s = S.EulerSolver(config_for(precision=prec, freestream=FS, cfl=0.4, local_time_stepping=True), mesh, U0=U0)
+        s.advance(2)
+        out[prec] = s.get_solver_data().get_solution()
+        s.close()
+    assert rel_linf(out[precision], out["fp64_ref"]) <= tol
+
+
+def test_separate_ghost_kernel_and_the_stage_kernels_ghosts_agree():
+    """advance() with the ghosts left by the stage kernel, against nf_stage with a halo unpack before
+    every stage (which has the ghost kernel compute them): the same bits."""
+    import ctypes as C
+
+    import torch
+
+    from netflux_b200 import _lib as L
+    m = _mesh((6, 4, 4), "all")
+    mesh = S.Mesh.from_tet_mesh(m)
+    U0 = _state(m)
+    out = []
+    for unpack in (False, True):
+        s = S.EulerSolver(config_for(precision="fp64", freestream=FS, cfl=0.4, local_time_stepping=True), mesh, U0=U0)
+        for _ in range(3):
+            s.calc_timestep(s.config)
+            for k in range(3):
+                if unpack:  # one cell's rows back into their own place
+                    cell = torch.zeros(1, dtype=torch.int64, device="cuda")
+                    buf = torch.zeros(10, dtype=torch.float64, device="cuda")
+                    p, b = C.cast(cell.data_ptr(), C.POINTER(C.c_int64)), C.cast(buf.data_ptr(), C.POINTER(C.c_double))
+                    assert L.load().nf_halo_pack(s._h, p, 1, b) == L.NF_OK
+                    assert L.load().nf_halo_unpack(s._h, p, 1, b) == L.NF_OK
+                assert L.load().nf_stage(s._h, k) == L.NF_OK
+        out.append(s.get_solver_data().get_solution())
+        s.close()
+    assert np.array_equal(out[0], out[1])
+
+
 def test_kept_fields_on_unlisted_faces():
     """The gradient and limiter fields of the FP64 form, with faces missing, against the reference order."""
     m = _mesh((5, 4, 3), "some")
