@@ -13,8 +13,8 @@
 //   mlp_backward_kernel    the same structure backwards (transposed weights,
 //                          SiLU derivative in the epilogue) -> dZ of each layer
 //   mlp_wgrad_kernel       dW = dZ^T H over the batch (split over CTAs), batch
-//                          chunks transposed while staged into one of two
-//                          operand buffers as the other's MMAs run, five
+//                          chunks copied as they are (MN-major operands) into
+//                          one of three buffers as another's MMAs run, five
 //                          accumulators in TMEM, bias gradients through a
 //                          column of ones
 //   mlp_adam_kernel        sums the per-CTA partial gradients, Adam update of
@@ -438,150 +438,110 @@ struct WgArgs {
   unsigned* status;
 };
 
-constexpr int WG_A = H * KC * 2;      // one [128 x KC] operand
-constexpr int WG_BA = NAUG * KC * 2;  // one [144 x KC] operand
-constexpr int WG_B16 = 16 * KC * 2;   // one [16 x KC] operand
+// Operands of a chunk of KC batch rows, MN-major (umma.cuh): the batch is K, and
+// the activations and gradients lie [batch][feature] in global memory, so each
+// 16-byte piece of a row (8 features) goes to its place in shared memory as it
+// is. 16 bytes between the 8-feature groups put a row's pieces on different banks.
+constexpr uint32_t WG_STRIDE = KC * 16 + 16;     // bytes between 8-feature groups
+constexpr int WG_A = (H / 8) * WG_STRIDE;        // one [128 x KC] operand
+constexpr int WG_BA = (NAUG / 8) * WG_STRIDE;    // one [144 x KC] operand
+constexpr int WG_B16 = 2 * WG_STRIDE;            // one [16 x KC] operand
 constexpr int WG_BUF = 5 * WG_A + 3 * WG_BA + 2 * WG_B16;  // one chunk's operands
 constexpr int WG_THREADS = 256;
-constexpr int WG_SMEM = 2 * WG_BUF + 64;  // two chunks: one staged while the other's MMAs run
+constexpr int WG_BUFS = 3;  // chunks in shared memory: one multiplied, two arriving
+constexpr int WG_SMEM = WG_BUFS * WG_BUF + 64;
 // TMEM columns of the five accumulators (32-column aligned; 512 allocated)
 constexpr int ACC1 = 0, ACC2 = 160, ACC3 = 320, ACC0 = 480, ACC4 = 496;
 
-// Column q (0..7) of an 8 x 8 BF16 block held as 8 rows of 16 bytes: the 8
-// values of that column as 16 bytes (row 0 first).
-__device__ __forceinline__ uint4 column8(const uint4 v[8], int q) {
-  const uint32_t sel = (q & 1) ? 0x7632u : 0x5410u;  // high or low 16-bit half of each word
-  uint32_t w[8];
-#pragma unroll
-  for (int r = 0; r < 8; r++) w[r] = (&v[r].x)[q >> 1];
-  uint4 o;
-  o.x = __byte_perm(w[0], w[1], sel);
-  o.y = __byte_perm(w[2], w[3], sel);
-  o.z = __byte_perm(w[4], w[5], sel);
-  o.w = __byte_perm(w[6], w[7], sel);
-  return o;
-}
-
-// rows [0, F) of a K-major [rows x KC] tile <- transpose of a [KC][F] row-major
-// BF16 block (batch rows b0 .. b0+KC; rows past B are zero). Each task is one
-// 8-feature chunk of 8 consecutive batch rows: eight 16-byte loads, an 8 x 8
-// transpose in registers, eight 16-byte stores of core-matrix rows.
-template <int F>
-__device__ __forceinline__ void stage_t(uint8_t* dst, const __nv_bfloat16* src, int64_t b0, int64_t B) {
-  constexpr int kChunks = F / 8, kTasks = kChunks * (KC / 8);
-  for (int task = threadIdx.x; task < kTasks; task += blockDim.x) {
-    const int ch = task % kChunks, rg = task / kChunks;
-    uint4 v[8];
-#pragma unroll
-    for (int r = 0; r < 8; r++) {
-      const int64_t b = b0 + rg * 8 + r;
-      v[r] = b < B ? *reinterpret_cast<const uint4*>(src + b * F + ch * 8) : make_uint4(0u, 0u, 0u, 0u);
-    }
-#pragma unroll
-    for (int q = 0; q < 8; q++)
-      *reinterpret_cast<uint4*>(dst + umma::kmaj_off(ch * 8 + q, rg * 8, KC)) = column8(v, q);
-  }
-}
-__device__ __forceinline__ void stage_t16(uint8_t* dst, const __nv_bfloat16* src, int64_t b0, int64_t B) {
-  stage_t<16>(dst, src, b0, B);
-}
-
 struct WgBuf {
-  uint8_t* A[5];  // dZ0^T, dZ1^T, dZ2^T, dZ3^T, H3^T
-  uint8_t* B[3];  // [H0|1]^T, [H1|1]^T, [H2|1]^T
-  uint8_t* X;     // X0^T
-  uint8_t* D4;    // dZ4^T
-  uint8_t* base;
-  __device__ explicit WgBuf(uint8_t* base_) : base(base_) {
-    for (int i = 0; i < 5; i++) A[i] = base + i * WG_A;
-    for (int i = 0; i < 3; i++) B[i] = base + 5 * WG_A + i * WG_BA;
-    X = base + 5 * WG_A + 3 * WG_BA;
-    D4 = X + WG_B16;
+  uint32_t base;  // shared-memory byte address
+  // operands in order: dZ0, dZ1, dZ2, dZ3, H3 (128 features each), [H0|1], [H1|1],
+  // [H2|1] (144), X0, dZ4 (16)
+  static __device__ constexpr uint32_t offset(int op) {
+    return op <= 5 ? uint32_t(op) * WG_A
+           : op <= 8 ? uint32_t(5 * WG_A + (op - 5) * WG_BA) : uint32_t(5 * WG_A + 3 * WG_BA + WG_B16);
   }
-  // the chunk of KC batch rows from b0, transposed into K-major operands. The
-  // tasks of the eight 128-feature operands (one 8-feature chunk of 8 rows
-  // each) are spread over all threads, two per thread with both tasks' loads
-  // issued before either's stores, so no thread runs the operands one after
-  // another while the others wait at the barrier.
-  __device__ void stage(const WgArgs& a, int64_t b0) {
-    constexpr int kPer = (H / 8) * (KC / 8), kWide = 8 * kPer;
-    static_assert(kWide == 2 * WG_THREADS, "two wide tasks per thread");
-    uint4 v[2][8];
-    int ch[2], rg[2];
-    uint8_t* dst[2];
+  // ask for the chunk of KC batch rows from b0 (rows past B are zero): 16
+  // pieces of 16 bytes a thread for the wide operands, half a piece for the narrow
+  __device__ void copy(const WgArgs& a, int64_t b0) const {
 #pragma unroll
-    for (int u = 0; u < 2; u++) {
-      const int task = threadIdx.x + u * WG_THREADS, op = task / kPer, lt = task % kPer;
-      ch[u] = lt % (H / 8);
-      rg[u] = lt / (H / 8);
-      // operands 0-3: dZ0..dZ3; 4: H3; 5-7: H0..H2
+    for (int op = 0; op < 8; op++) {
       const __nv_bfloat16* src = op < 4 ? a.dz + int64_t(op) * a.B * H : a.save + save_h(a.B, op == 4 ? 3 : op - 5);
-      dst[u] = op < 5 ? base + op * WG_A : base + 5 * WG_A + (op - 5) * WG_BA;  // A[op] or B[op - 5]
 #pragma unroll
-      for (int r = 0; r < 8; r++) {
-        const int64_t b = b0 + rg[u] * 8 + r;
-        v[u][r] = b < a.B ? *reinterpret_cast<const uint4*>(src + b * H + ch[u] * 8) : make_uint4(0u, 0u, 0u, 0u);
+      for (int u = 0; u < KC * (H / 8) / WG_THREADS; u++) {
+        const int piece = threadIdx.x + u * WG_THREADS, k = piece / (H / 8), f8 = piece % (H / 8);
+        const int64_t b = b0 + k;
+        const bool valid = b < a.B;
+        umma::copy16_async(base + offset(op) + umma::mnmaj_off(f8, k, WG_STRIDE), src + (valid ? b : 0) * H + f8 * 8,
+                           valid);
       }
     }
-#pragma unroll
-    for (int u = 0; u < 2; u++)
-#pragma unroll
-      for (int q = 0; q < 8; q++)
-        *reinterpret_cast<uint4*>(dst[u] + umma::kmaj_off(ch[u] * 8 + q, rg[u] * 8, KC)) = column8(v[u], q);
-    stage_t16(X, a.save + save_x0(a.B), b0, a.B);
-    stage_t16(D4, a.dz4, b0, a.B);
+    if (threadIdx.x < 4 * KC) {
+      const int op = threadIdx.x / (2 * KC), k = threadIdx.x / 2 % KC, f8 = threadIdx.x % 2;
+      const int64_t b = b0 + k;
+      const bool valid = b < a.B;
+      const __nv_bfloat16* src = op == 0 ? a.save + save_x0(a.B) : a.dz4;
+      umma::copy16_async(base + offset(8 + op) + umma::mnmaj_off(f8, k, WG_STRIDE), src + (valid ? b : 0) * 16 + f8 * 8,
+                         valid);
+    }
   }
+  __device__ uint64_t desc(int op, int s) const { return umma::mnmaj_desc(base + offset(op), WG_STRIDE, s); }
   // every accumulator += this chunk's product (one thread)
   __device__ void issue(uint32_t tbase, bool first) const {
-    const uint32_t idA = umma::idesc_bf16(128, NAUG), id16 = umma::idesc_bf16(128, 16);
+    const uint32_t idA = umma::idesc_bf16_mn(128, NAUG), id16 = umma::idesc_bf16_mn(128, 16);
 #pragma unroll 1
     for (int s = 0; s < KC / 16; s++) {
       const uint32_t acc = (first && s == 0) ? 0u : 1u;
-#pragma unroll
-      for (int l = 1; l <= 3; l++)
-        umma::mma_bf16(tbase + uint32_t(l == 1 ? ACC1 : l == 2 ? ACC2 : ACC3),
-                       umma::kmaj_desc(umma::smem_addr(A[l]), KC, s), umma::kmaj_desc(umma::smem_addr(B[l - 1]), KC, s),
-                       idA, acc);
-      umma::mma_bf16(tbase + ACC0, umma::kmaj_desc(umma::smem_addr(A[0]), KC, s),
-                     umma::kmaj_desc(umma::smem_addr(X), KC, s), id16, acc);
-      umma::mma_bf16(tbase + ACC4, umma::kmaj_desc(umma::smem_addr(A[4]), KC, s),
-                     umma::kmaj_desc(umma::smem_addr(D4), KC, s), id16, acc);
+      umma::mma_bf16(tbase + ACC1, desc(1, s), desc(5, s), idA, acc);
+      umma::mma_bf16(tbase + ACC2, desc(2, s), desc(6, s), idA, acc);
+      umma::mma_bf16(tbase + ACC3, desc(3, s), desc(7, s), idA, acc);
+      umma::mma_bf16(tbase + ACC0, desc(0, s), desc(8, s), id16, acc);
+      umma::mma_bf16(tbase + ACC4, desc(4, s), desc(9, s), id16, acc);
     }
   }
 };
 
-// The CTA's chunks in turn through two operand buffers: while the tensor core
-// multiplies chunk i from one buffer, the threads stage chunk i + 1 into the
-// other (after the MMAs of chunk i - 1, which read it, are done).
+// The CTA's chunks in turn through three operand buffers: while the tensor core
+// multiplies chunk i, chunks i + 1 and i + 2 are on their way (131 KB a CTA).
+// Reads 2.1 KB a sample once; at 65,536 samples 59 us (2.4 TB/s), 121 us with
+// chunks transposed through registers into two buffers.
 __global__ void __launch_bounds__(WG_THREADS, 1) mlp_wgrad_kernel(WgArgs a) {
   extern __shared__ __align__(1024) uint8_t sm[];
-  uint64_t* s_mbar = reinterpret_cast<uint64_t*>(sm + 2 * WG_BUF);  // one per buffer
-  uint32_t* s_tslot = reinterpret_cast<uint32_t*>(s_mbar + 2);
+  uint64_t* s_mbar = reinterpret_cast<uint64_t*>(sm + WG_BUFS * WG_BUF);  // one per buffer
+  uint32_t* s_tslot = reinterpret_cast<uint32_t*>(s_mbar + WG_BUFS);
   const int t = threadIdx.x;
-  // constant rows of the augmented operands: a row of ones, then zeros
-  for (int task = t; task < 2 * 3 * (NAUG - H) * (KC / 8); task += blockDim.x) {
-    const int g = task % (KC / 8), r = H + (task / (KC / 8)) % (NAUG - H), i = task / (KC / 8) / (NAUG - H);
-    float v[8];
-#pragma unroll
-    for (int j = 0; j < 8; j++) v[j] = r == H ? 1.f : 0.f;
-    uint8_t* op = sm + (i / 3) * WG_BUF + 5 * WG_A + (i % 3) * WG_BA;  // WgBuf::B[i % 3] of buffer i / 3
-    *reinterpret_cast<uint4*>(op + umma::kmaj_off(r, g * 8, KC)) = pack8(v);
-  }
-  const uint32_t tbase = setup(s_mbar, 2, s_tslot, 512);
-  TileSync sync0{umma::smem_addr(s_mbar), 0u, a.status}, sync1{umma::smem_addr(s_mbar + 1), 0u, a.status};
-  auto wait_buf = [&](int k) { return k == 0 ? sync0.wait() : sync1.wait(); };
+  const uint32_t sm0 = umma::smem_addr(sm);
   const int64_t n_chunks = (a.B + KC - 1) / KC;
+  auto buf = [&](int k) { return WgBuf{sm0 + uint32_t(k) * WG_BUF}; };
+  // chunks blockIdx.x, + gridDim.x, ...; the first two asked for before anything else
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    const int64_t ch = int64_t(blockIdx.x) + int64_t(k) * gridDim.x;
+    if (ch < n_chunks) buf(k).copy(a, ch * KC);
+    umma::copy_commit();
+  }
+  // constant rows of the augmented operands: a row of ones, then zeros
+  for (int task = t; task < WG_BUFS * 3 * 2 * KC; task += blockDim.x) {
+    const int k = task % KC, f8 = H / 8 + task / KC % 2, i = task / (2 * KC);
+    *reinterpret_cast<uint4*>(sm + (i / 3) * WG_BUF + WgBuf::offset(5 + i % 3) + umma::mnmaj_off(f8, k, WG_STRIDE)) =
+        make_uint4(f8 == H / 8 ? 0x3f80u : 0u, 0u, 0u, 0u);  // BF16 1, or zeros
+  }
+  const uint32_t tbase = setup(s_mbar, WG_BUFS, s_tslot, 512);
+  TileSync sync[WG_BUFS];
+#pragma unroll
+  for (int k = 0; k < WG_BUFS; k++) sync[k] = TileSync{umma::smem_addr(s_mbar + k), 0u, a.status};
+  auto wait_buf = [&](int k) { return k == 0 ? sync[0].wait() : k == 1 ? sync[1].wait() : sync[2].wait(); };
   float db4 = 0.f;
   int i = 0;  // chunks of this CTA issued
-  if (int64_t(blockIdx.x) < n_chunks) WgBuf(sm).stage(a, int64_t(blockIdx.x) * KC);
-  umma::fence_async_shared();
-  __syncthreads();
   for (int64_t ch = blockIdx.x; ch < n_chunks; ch += gridDim.x, i++) {
-    const int cur = i & 1;
+    const int cur = i % WG_BUFS;
+    umma::copy_wait<1>();  // this thread's pieces of chunk i are here
+    umma::fence_async_shared();
+    __syncthreads();
     if (t == 0) {
       umma::fence_after_sync();
-      WgBuf(sm + cur * WG_BUF).issue(tbase, i == 0);
-      umma::commit(cur == 0 ? sync0.mbar : sync1.mbar);
+      buf(cur).issue(tbase, i == 0);
+      umma::commit(umma::smem_addr(s_mbar + cur));
     }
     // bias gradient of the output layer: this thread's output t & 15 over the chunk's rows
     // t >> 4 and (t >> 4) + 16 (two independent loads, no thread waits on a serial sum)
@@ -590,15 +550,13 @@ __global__ void __launch_bounds__(WG_THREADS, 1) mlp_wgrad_kernel(WgArgs a) {
       const int64_t b = ch * KC + j;
       if (b < a.B) db4 += __bfloat162float(a.dz4[b * 16 + (t & 15)]);
     }
-    const int64_t nx = ch + gridDim.x;
-    if (nx < n_chunks) {
-      if (i >= 1 && !wait_buf(cur ^ 1)) goto done;  // chunk i - 1 has read the other buffer
-      WgBuf(sm + (cur ^ 1) * WG_BUF).stage(a, nx * KC);
-      umma::fence_async_shared();
-    }
-    __syncthreads();  // the next chunk's operands staged before it is issued
+    const int64_t nx = ch + 2 * int64_t(gridDim.x);
+    if (i >= 1 && !wait_buf((i - 1) % WG_BUFS)) goto done;  // chunk i - 1 has left the buffer of chunk i + 2
+    if (nx < n_chunks) buf((i + 2) % WG_BUFS).copy(a, nx * KC);
+    umma::copy_commit();
   }
-  if (i > 0 && !wait_buf((i - 1) & 1)) goto done;  // the last chunk, and with it every earlier one
+  umma::copy_wait<0>();
+  if (i > 0 && !wait_buf((i - 1) % WG_BUFS)) goto done;  // the last chunk, and with it every earlier one
   {
     float* P = a.partial + int64_t(blockIdx.x) * N_PARAM;
     const int row = t & 127, half = t >> 7;  // TMEM lane; which accumulators this warpgroup reads
@@ -606,6 +564,9 @@ __global__ void __launch_bounds__(WG_THREADS, 1) mlp_wgrad_kernel(WgArgs a) {
     if (i == 0) {  // this CTA had no rows
       for (int k = t; k < N_PARAM; k += blockDim.x) P[k] = 0.f;
     } else {
+      auto store4 = [](float* p, const float* v, int n) {  // 16-byte stores (every row starts on 16 bytes)
+        for (int j = 0; j < n; j += 4) *reinterpret_cast<float4*>(p + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+      };
       for (int l = 1 + half; l <= 3; l += 2) {  // layers 1, 3 | 2
         const uint32_t base = lane_addr + uint32_t(l == 1 ? ACC1 : l == 2 ? ACC2 : ACC3);
         const int offW = l == 1 ? OFF_W1 : l == 2 ? OFF_W2 : OFF_W3;
@@ -614,8 +575,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) mlp_wgrad_kernel(WgArgs a) {
         for (int c0 = 0; c0 < H; c0 += 32) {
           float v[32];
           umma::tmem_ld32(base + uint32_t(c0), v);
-#pragma unroll
-          for (int j = 0; j < 32; j++) P[offW + row * H + c0 + j] = v[j];
+          store4(P + offW + row * H + c0, v, 32);
         }
         float v[16];
         umma::tmem_ld16(base + uint32_t(H), v);
@@ -624,8 +584,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) mlp_wgrad_kernel(WgArgs a) {
       if (half == 1) {
         float v[16];
         umma::tmem_ld16(lane_addr + ACC0, v);
-#pragma unroll
-        for (int j = 0; j < 16; j++) P[OFF_W0 + row * KIN + j] = v[j];
+        store4(P + OFF_W0 + row * KIN, v, 16);
         umma::tmem_ld16(lane_addr + ACC4, v);
 #pragma unroll
         for (int j = 0; j < 16; j++) P[OFF_W4 + j * H + row] = v[j];
@@ -644,6 +603,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) mlp_wgrad_kernel(WgArgs a) {
     }
   }
 done:
+  umma::copy_wait<0>();  // no copy may land after the block has left
   teardown(tbase, 512);
 }
 

@@ -35,9 +35,39 @@ __device__ __forceinline__ uint64_t kmaj_desc(uint32_t base, int K, int s) {
   return (start & 0x3FFFull) | ((lbo & 0x3FFFull) << 16) | ((sbo & 0x3FFFull) << 32) | (1ull << 46);
 }
 
+// MN-major operand (M or N contiguous, no swizzle): the tile is a grid of 8 (MN,
+// 16 contiguous bytes) x 8 (K, 16 bytes apart) core matrices of 128 bytes; core
+// matrices adjacent in K are 128 bytes apart (leading byte offset), those
+// adjacent in MN `mn_stride` bytes (stride byte offset; any multiple of 16).
+// A row-major [K][MN] block in global memory is copied into it 16 bytes at a time
+// without a transpose.
+__device__ __forceinline__ uint32_t mnmaj_off(int mn8, int k, uint32_t mn_stride) {
+  return uint32_t(mn8) * mn_stride + uint32_t(k) * 16u;
+}
+// descriptor of the K-slice [16 s, 16 s + 16) of such a tile at smem byte address base
+__device__ __forceinline__ uint64_t mnmaj_desc(uint32_t base, uint32_t mn_stride, int s) {
+  const uint64_t start = (base + uint32_t(s) * 256u) >> 4;
+  const uint64_t lbo = 128u >> 4;
+  const uint64_t sbo = mn_stride >> 4;
+  return (start & 0x3FFFull) | ((lbo & 0x3FFFull) << 16) | ((sbo & 0x3FFFull) << 32) | (1ull << 46);
+}
+
 // kind::f16 instruction descriptor: D FP32, A and B BF16, both K-major
 __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
   return (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(N >> 3) << 17) | (uint32_t(M >> 4) << 24);
+}
+// the same, both operands MN-major
+__host__ __device__ constexpr uint32_t idesc_bf16_mn(int M, int N) { return idesc_bf16(M, N) | (1u << 15) | (1u << 16); }
+
+// 16 bytes from global to shared memory without a register; zeros where !valid
+// (src is not read then, but must be an address)
+__device__ __forceinline__ void copy16_async(uint32_t dst, const void* src, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int kPending>
+__device__ __forceinline__ void copy_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory");
 }
 
 // D[tmem] (+)= A * B^T for one K = 16 step, issued by one thread
