@@ -99,6 +99,17 @@ __device__ __forceinline__ uint4 pack8(const float* v) {
   }
   return r;
 }
+// 32 bytes, one full sector, to or from a 32-byte aligned address
+__device__ __forceinline__ void store32(void* p, uint4 a, uint4 b) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(a.x), "r"(a.y), "r"(a.z),
+               "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
+               : "memory");
+}
+__device__ __forceinline__ void load32(const void* p, uint4& a, uint4& b) {
+  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
+               : "l"(p));
+}
 __device__ __forceinline__ void unpack8(uint4 r, float* v) {
   const uint32_t* w = reinterpret_cast<const uint32_t*>(&r);
 #pragma unroll
@@ -111,26 +122,34 @@ __device__ __forceinline__ void unpack8(uint4 r, float* v) {
 }
 
 // Tiles in flight per CTA in the forward and backward kernels: each has its
-// own 128 threads (one warpgroup), operand buffers, mbarrier and TMEM
-// accumulator, so one tile's MMAs run while another's epilogue does.
+// own operand buffers, mbarrier and TMEM accumulator, so one tile's MMAs run
+// while another's epilogue does, and its own two warpgroups, which take half of
+// the columns of each row in the epilogues, what these kernels spend their time on
+// (128 threads a tile: forward 97 us at 65,536 samples, backward 134; 256: 102 and
+// 87; with whole 32-byte sectors stored and loaded by a thread, not halves, 75 and
+// 81; prediction, which stores nothing between the layers, of 1M samples 0.86 ->
+// 0.65 ms).
 constexpr int NSLOT = 2;
+constexpr int SLOT_THREADS = 256;
 // CTAs that give every slot at least one tile of B samples
 inline int tile_ctas(int64_t B) { return int(((B + TILE - 1) / TILE + NSLOT - 1) / NSLOT); }
 
-// Barrier among the 128 threads of one slot (named barriers 1..NSLOT; 0 is
+// Barrier among the threads of one slot (named barriers 1..NSLOT; 0 is
 // __syncthreads), optionally AND-reducing a predicate over them.
-__device__ __forceinline__ void slot_sync(int slot) { asm volatile("bar.sync %0, 128;" ::"r"(slot + 1) : "memory"); }
+__device__ __forceinline__ void slot_sync(int slot) {
+  asm volatile("bar.sync %0, %1;" ::"r"(slot + 1), "n"(SLOT_THREADS) : "memory");
+}
 __device__ __forceinline__ bool slot_sync_and(int slot, bool v) {
   uint32_t r;
   asm volatile(
       "{\n\t"
       ".reg .pred p, q;\n\t"
       "setp.ne.u32 q, %1, 0;\n\t"
-      "bar.red.and.pred p, %2, 128, q;\n\t"
+      "bar.red.and.pred p, %2, %3, q;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t"
       "}\n"
       : "=r"(r)
-      : "r"(uint32_t(v)), "r"(slot + 1)
+      : "r"(uint32_t(v)), "r"(slot + 1), "n"(SLOT_THREADS)
       : "memory");
   return r != 0;
 }
@@ -139,7 +158,7 @@ struct TileSync {
   uint32_t mbar;
   uint32_t phase = 0;
   unsigned* status;
-  int slot = -1;  // -1: the whole CTA takes part; else the slot's 128 threads
+  int slot = -1;  // -1: the whole CTA takes part; else the slot's threads
   // wait for the MMAs committed to mbar; every participating thread agrees on
   // the outcome
   __device__ bool wait() {
@@ -192,9 +211,10 @@ struct FwdArgs {
 constexpr int FWD_SLOT = TILE * H * 2 + TILE * KIN * 2;  // one tile's activations and inputs
 constexpr int FWD_SMEM = IMG_FWD + NSLOT * FWD_SLOT + (3 * H + NOUT) * 4 + 64;
 
-__global__ void __launch_bounds__(128 * NSLOT, 1) mlp_forward_kernel(FwdArgs a) {
+__global__ void __launch_bounds__(SLOT_THREADS * NSLOT, 1) mlp_forward_kernel(FwdArgs a) {
   extern __shared__ __align__(1024) uint8_t sm[];
-  const int slot = threadIdx.x >> 7, t = threadIdx.x & 127, w = t >> 5;
+  // this thread's row of the tile and its half of the columns
+  const int slot = threadIdx.x / SLOT_THREADS, t = threadIdx.x & 127, half = threadIdx.x >> 7 & 1, w = t >> 5;
   uint8_t* s_img = sm;
   uint8_t* s_act = sm + IMG_FWD + slot * FWD_SLOT;  // [128 x K128] activations of this slot's tile
   uint8_t* s_x0 = s_act + TILE * H * 2;             // [128 x K16] inputs
@@ -219,7 +239,7 @@ __global__ void __launch_bounds__(128 * NSLOT, 1) mlp_forward_kernel(FwdArgs a) 
   for (int64_t tile = int64_t(blockIdx.x) * NSLOT + slot; tile < n_tiles; tile += int64_t(gridDim.x) * NSLOT) {
     const int64_t b = tile * TILE + t;
     const bool valid = b < a.B;
-    {  // inputs: 7 features, a constant 1 (bias of layer 0), zeros
+    if (half == 0) {  // inputs: 7 features, a constant 1 (bias of layer 0), zeros
       float x[KIN];
 #pragma unroll
       for (int k = 0; k < KIN; k++) x[k] = 0.f;
@@ -241,7 +261,7 @@ __global__ void __launch_bounds__(128 * NSLOT, 1) mlp_forward_kernel(FwdArgs a) 
     umma::fence_async_shared();
     slot_sync(slot);
     for (int l = 0; l < 5; l++) {
-      if (t == 0) {
+      if (t == 0 && half == 0) {
         umma::fence_after_sync();
         if (l == 0) {
           umma::mma_bf16(tacc, umma::kmaj_desc(a_x0, KIN, 0), umma::kmaj_desc(a_img + IMG_W0, KIN, 0), id128, 0);
@@ -258,26 +278,33 @@ __global__ void __launch_bounds__(128 * NSLOT, 1) mlp_forward_kernel(FwdArgs a) 
       if (l < 4) {
         // z = acc (+ bias), h = silu(z): the next layer's operand
 #pragma unroll 1
-        for (int c0 = 0; c0 < H; c0 += 32) {
-          float v[32];
-          umma::tmem_ld32(lane_addr + uint32_t(c0), v);
+        for (int c0 = half * (H / 2); c0 < (half + 1) * (H / 2); c0 += 32) {
           float z[32], h[32];
+          umma::tmem_ld32(lane_addr + uint32_t(c0), z);
+          if (l > 0) {
 #pragma unroll
-          for (int j = 0; j < 32; j++) {
-            z[j] = l == 0 ? v[j] : v[j] + s_bias[(l - 1) * H + c0 + j];
-            h[j] = silu(z[j]);
+            for (int j = 0; j < 32; j += 4) {
+              const float4 b4 = *reinterpret_cast<const float4*>(s_bias + (l - 1) * H + c0 + j);
+              z[j] += b4.x;
+              z[j + 1] += b4.y;
+              z[j + 2] += b4.z;
+              z[j + 3] += b4.w;
+            }
           }
 #pragma unroll
-          for (int q = 0; q < 4; q++) {
-            const uint4 hv = pack8(h + 8 * q);
-            *reinterpret_cast<uint4*>(s_act + umma::kmaj_off(t, c0 + 8 * q, H)) = hv;
+          for (int j = 0; j < 32; j++) h[j] = silu(z[j]);
+#pragma unroll
+          for (int q = 0; q < 4; q += 2) {
+            const uint4 h0 = pack8(h + 8 * q), h1 = pack8(h + 8 * q + 8);
+            *reinterpret_cast<uint4*>(s_act + umma::kmaj_off(t, c0 + 8 * q, H)) = h0;
+            *reinterpret_cast<uint4*>(s_act + umma::kmaj_off(t, c0 + 8 * q + 8, H)) = h1;
             if (a.save && valid) {
-              *reinterpret_cast<uint4*>(a.save + save_z(a.B, l) + b * H + c0 + 8 * q) = pack8(z + 8 * q);
-              *reinterpret_cast<uint4*>(a.save + save_h(a.B, l) + b * H + c0 + 8 * q) = hv;
+              store32(a.save + save_z(a.B, l) + b * H + c0 + 8 * q, pack8(z + 8 * q), pack8(z + 8 * q + 8));
+              store32(a.save + save_h(a.B, l) + b * H + c0 + 8 * q, h0, h1);
             }
           }
         }
-      } else {
+      } else if (half == 0) {
         float v[16];
         umma::tmem_ld16(lane_addr, v);
         float y[NO];
@@ -336,9 +363,10 @@ struct BwdArgs {
 constexpr int BWD_SLOT = TILE * H * 2 + TILE * NOUT * 2;  // one tile's operand and output gradient
 constexpr int BWD_SMEM = IMG_BWD + NSLOT * BWD_SLOT + 64;
 
-__global__ void __launch_bounds__(128 * NSLOT, 1) mlp_backward_kernel(BwdArgs a) {
+__global__ void __launch_bounds__(SLOT_THREADS * NSLOT, 1) mlp_backward_kernel(BwdArgs a) {
   extern __shared__ __align__(1024) uint8_t sm[];
-  const int slot = threadIdx.x >> 7, t = threadIdx.x & 127, w = t >> 5;
+  // this thread's row of the tile and its half of the columns
+  const int slot = threadIdx.x / SLOT_THREADS, t = threadIdx.x & 127, half = threadIdx.x >> 7 & 1, w = t >> 5;
   uint8_t* s_img = sm;
   uint8_t* s_act = sm + IMG_BWD + slot * BWD_SLOT;
   uint8_t* s_d4 = s_act + TILE * H * 2;
@@ -359,7 +387,7 @@ __global__ void __launch_bounds__(128 * NSLOT, 1) mlp_backward_kernel(BwdArgs a)
   for (int64_t tile = int64_t(blockIdx.x) * NSLOT + slot; tile < n_tiles; tile += int64_t(gridDim.x) * NSLOT) {
     const int64_t b = tile * TILE + t;
     const bool valid = b < a.B;
-    {
+    if (half == 0) {
       uint4 c0 = make_uint4(0, 0, 0, 0), c1 = c0;
       if (valid) {
         const uint4* g = reinterpret_cast<const uint4*>(a.dz4 + b * NOUT);
@@ -373,7 +401,7 @@ __global__ void __launch_bounds__(128 * NSLOT, 1) mlp_backward_kernel(BwdArgs a)
     slot_sync(slot);
     // layer l's input gradient: dH_{l-1} = dZ_l W_l, then dZ_{l-1} = dH_{l-1} silu'(Z_{l-1})
     for (int l = 4; l >= 1; l--) {
-      if (t == 0) {
+      if (t == 0 && half == 0) {
         umma::fence_after_sync();
         if (l == 4) {
           umma::mma_bf16(tacc, umma::kmaj_desc(a_d4, NOUT, 0), umma::kmaj_desc(a_img + IMG_T4, NOUT, 0), id128, 0);
@@ -392,27 +420,35 @@ __global__ void __launch_bounds__(128 * NSLOT, 1) mlp_backward_kernel(BwdArgs a)
       const __nv_bfloat16* zrow = a.save + save_z(a.B, lo) + b * H;
       auto load_z = [&](uint4* z4, int c0) {
 #pragma unroll
-        for (int q = 0; q < 4; q++)
-          z4[q] = valid ? *reinterpret_cast<const uint4*>(zrow + c0 + 8 * q) : make_uint4(0u, 0u, 0u, 0u);
+        for (int q = 0; q < 4; q += 2) {
+          z4[q] = z4[q + 1] = make_uint4(0u, 0u, 0u, 0u);
+          if (valid) load32(zrow + c0 + 8 * q, z4[q], z4[q + 1]);
+        }
       };
+      const int c_end = (half + 1) * (H / 2);
       uint4 zc[4];
-      load_z(zc, 0);
+      load_z(zc, half * (H / 2));
       if (!sync.wait()) goto done;
 #pragma unroll 1
-      for (int c0 = 0; c0 < H; c0 += 32) {
+      for (int c0 = half * (H / 2); c0 < c_end; c0 += 32) {
         uint4 zn[4];
-        if (c0 + 32 < H) load_z(zn, c0 + 32);
+        if (c0 + 32 < c_end) load_z(zn, c0 + 32);
         float v[32];
         umma::tmem_ld32(lane_addr + uint32_t(c0), v);
+        uint4 dv[4];
 #pragma unroll
         for (int q = 0; q < 4; q++) {
           float z[8], d[8];
           unpack8(zc[q], z);
 #pragma unroll
           for (int j = 0; j < 8; j++) d[j] = valid ? v[8 * q + j] * dsilu(z[j]) : 0.f;
-          const uint4 dv = pack8(d);
-          *reinterpret_cast<uint4*>(s_act + umma::kmaj_off(t, c0 + 8 * q, H)) = dv;
-          if (valid) *reinterpret_cast<uint4*>(a.dz + int64_t(lo) * a.B * H + b * H + c0 + 8 * q) = dv;
+          dv[q] = pack8(d);
+          *reinterpret_cast<uint4*>(s_act + umma::kmaj_off(t, c0 + 8 * q, H)) = dv[q];
+        }
+        if (valid) {
+          __nv_bfloat16* dz = a.dz + int64_t(lo) * a.B * H + b * H + c0;
+          store32(dz, dv[0], dv[1]);
+          store32(dz + 16, dv[2], dv[3]);
         }
 #pragma unroll
         for (int q = 0; q < 4; q++) zc[q] = zn[q];
@@ -842,9 +878,9 @@ struct nf_mlp {
     fa.loss_scale = 2.0f / float(B * NO);
     fa.status = status.p;
     const int n_cta = std::min(tile_ctas(B), n_sm);
-    mlp_forward_kernel<<<n_cta, 128 * NSLOT, FWD_SMEM, stream>>>(fa);
+    mlp_forward_kernel<<<n_cta, SLOT_THREADS * NSLOT, FWD_SMEM, stream>>>(fa);
     BwdArgs ba{img_bwd.p, save.p, dz4.p, B, dz.p, status.p};
-    mlp_backward_kernel<<<n_cta, 128 * NSLOT, BWD_SMEM, stream>>>(ba);
+    mlp_backward_kernel<<<n_cta, SLOT_THREADS * NSLOT, BWD_SMEM, stream>>>(ba);
     WgArgs wa{save.p, dz.p, dz4.p, B, partial.p, status.p};
     mlp_wgrad_kernel<<<n_wg, WG_THREADS, WG_SMEM, stream>>>(wa);
     mlp_adam_kernel<<<(N_PARAM + 255) / 256, 256, 0, stream>>>(adam_args(lr, apply));
@@ -1070,7 +1106,7 @@ int nf_mlp_predict(nf_mlp* m, const float* features, int64_t n, float* out, doub
     ck(cudaEventCreate(&e0), "event");
     ck(cudaEventCreate(&e1), "event");
     ck(cudaEventRecord(e0, m->stream), "event");
-    mlp_forward_kernel<<<std::min(tile_ctas(n), m->n_sm), 128 * NSLOT, FWD_SMEM, m->stream>>>(fa);
+    mlp_forward_kernel<<<std::min(tile_ctas(n), m->n_sm), SLOT_THREADS * NSLOT, FWD_SMEM, m->stream>>>(fa);
     ck(cudaGetLastError(), "launch");
     ck(cudaEventRecord(e1, m->stream), "event");
     ck(cudaMemcpyAsync(out, o.p, size_t(n) * NO * sizeof(float), cudaMemcpyDeviceToHost, m->stream), "D2H");
