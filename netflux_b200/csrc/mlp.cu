@@ -756,28 +756,143 @@ __global__ void __launch_bounds__(128, 1) umma_gemm_test_kernel(const __nv_bfloa
 }
 
 // Distance from each point to the nearest of m wall points (the surrogate's
-// wall-distance input): one thread per point, wall points staged through
-// shared memory in tiles of 1024.
-constexpr int WD_TILE = 1024;
+// wall-distance input). The wall points lie in the order of the mesh's patches, so
+// 32 consecutive ones are close together (a cluster) and 32 clusters still are (a
+// group); points come in cell order, so a warp's 32 are close together too. A warp
+// passes over every group and cluster whose box is no nearer to its own points'
+// box than the farthest of its nearest distances so far. The bound is computed
+// with the operations of the distance itself on differences that are no larger,
+// and rounding is monotone, so no distance below a passed one is missed: the result
+// is the minimum over all points, bit for bit. Unordered points only pass over
+// less. 1.3M cells and 36,864 wall points, the whole call: 17 ms
+// over all pairs, 2.4 ms so (of which 1.4 ms are its copies).
+constexpr int WD_C = 32;  // points a cluster, clusters a group
+struct WallBox {
+  float4 lo, hi;
+};
+__device__ __forceinline__ float box_distance2(const WallBox& a, const WallBox& b) {
+  const float dx = fmaxf(fmaxf(a.lo.x - b.hi.x, b.lo.x - a.hi.x), 0.f);
+  const float dy = fmaxf(fmaxf(a.lo.y - b.hi.y, b.lo.y - a.hi.y), 0.f);
+  const float dz = fmaxf(fmaxf(a.lo.z - b.hi.z, b.lo.z - a.hi.z), 0.f);
+  return fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+}
+// the box of the warp's values in every lane (a lane without one passes an empty box)
+__device__ __forceinline__ WallBox warp_box(WallBox b) {
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    b.lo.x = fminf(b.lo.x, __shfl_xor_sync(0xffffffffu, b.lo.x, off));
+    b.lo.y = fminf(b.lo.y, __shfl_xor_sync(0xffffffffu, b.lo.y, off));
+    b.lo.z = fminf(b.lo.z, __shfl_xor_sync(0xffffffffu, b.lo.z, off));
+    b.hi.x = fmaxf(b.hi.x, __shfl_xor_sync(0xffffffffu, b.hi.x, off));
+    b.hi.y = fmaxf(b.hi.y, __shfl_xor_sync(0xffffffffu, b.hi.y, off));
+    b.hi.z = fmaxf(b.hi.z, __shfl_xor_sync(0xffffffffu, b.hi.z, off));
+  }
+  return b;
+}
+constexpr float kWallFar = 3.0e38f;
+__device__ __forceinline__ WallBox empty_box() {
+  return WallBox{make_float4(kWallFar, kWallFar, kWallFar, 0.f), make_float4(-kWallFar, -kWallFar, -kWallFar, 0.f)};
+}
+
+// One warp a cluster: its points as float4 (the last cluster filled up with its
+// last point) and its box.
+__global__ void __launch_bounds__(256) wall_cluster_kernel(const float* __restrict__ wall, int64_t m, int64_t n_clusters,
+                                                          float4* __restrict__ pt, WallBox* __restrict__ box) {
+  const int64_t c = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (c >= n_clusters) return;
+  const int64_t i = c * WD_C + lane < m ? c * WD_C + lane : m - 1;
+  const float4 p = make_float4(wall[3 * i], wall[3 * i + 1], wall[3 * i + 2], 0.f);
+  pt[c * WD_C + lane] = p;
+  const WallBox b = warp_box(WallBox{p, p});
+  if (lane == 0) box[c] = b;
+}
+// One warp a group: the box of its clusters.
+__global__ void __launch_bounds__(256) wall_group_kernel(const WallBox* __restrict__ box, int64_t n_clusters,
+                                                        int64_t n_groups, WallBox* __restrict__ group) {
+  const int64_t g = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (g >= n_groups) return;
+  const int64_t c = g * WD_C + lane;
+  const WallBox b = warp_box(c < n_clusters ? box[c] : empty_box());
+  if (lane == 0) group[g] = b;
+}
+
 __global__ void __launch_bounds__(256) wall_distance_kernel(const float* __restrict__ pts, int64_t n,
-                                                             const float* __restrict__ wall, int64_t m,
-                                                             float* __restrict__ out) {
-  __shared__ float sw[3 * WD_TILE];
+                                                            const float4* __restrict__ wall,
+                                                            const WallBox* __restrict__ box, int64_t n_clusters,
+                                                            const WallBox* __restrict__ group, int64_t n_groups,
+                                                            float* __restrict__ out) {
   const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  const float px = i < n ? pts[3 * i] : 0.f, py = i < n ? pts[3 * i + 1] : 0.f, pz = i < n ? pts[3 * i + 2] : 0.f;
-  float best = 3.0e38f;
-  for (int64_t t0 = 0; t0 < m; t0 += WD_TILE) {
-    const int cnt = int(m - t0 < WD_TILE ? m - t0 : WD_TILE);
-    __syncthreads();
-    for (int j = threadIdx.x; j < 3 * cnt; j += blockDim.x) sw[j] = wall[3 * t0 + j];
-    __syncthreads();
-#pragma unroll 4
-    for (int j = 0; j < cnt; j++) {
-      const float dx = px - sw[3 * j], dy = py - sw[3 * j + 1], dz = pz - sw[3 * j + 2];
+  const int lane = threadIdx.x & 31;
+  const bool in = i < n;
+  if (__ballot_sync(0xffffffffu, in) == 0) return;
+  const float px = in ? pts[3 * i] : 0.f, py = in ? pts[3 * i + 1] : 0.f, pz = in ? pts[3 * i + 2] : 0.f;
+  const float4 p = make_float4(px, py, pz, 0.f);
+  const WallBox mine = warp_box(in ? WallBox{p, p} : empty_box());
+  float best = in ? kWallFar : 0.f;  // a lane without a point asks for nothing
+  float limit = kWallFar;            // the largest best of the warp
+  auto visit = [&](int64_t c) {
+    const float4* w = wall + c * WD_C;
+#pragma unroll 8
+    for (int j = 0; j < WD_C; j++) {
+      const float4 q = w[j];
+      const float dx = px - q.x, dy = py - q.y, dz = pz - q.z;
       best = fminf(best, fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
     }
+    limit = best;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) limit = fmaxf(limit, __shfl_xor_sync(0xffffffffu, limit, off));
+  };
+  // the lane's candidate with the smallest bound, and where it is
+  auto nearest = [&](float d, int64_t at) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      const float od = __shfl_xor_sync(0xffffffffu, d, off);
+      const int64_t oa = __shfl_xor_sync(0xffffffffu, at, off);
+      if (od < d || (od == d && oa < at)) {
+        d = od;
+        at = oa;
+      }
+    }
+    return at;
+  };
+  // the cluster that looks nearest first, for a close limit
+  float d = kWallFar;
+  int64_t at = 0;
+  for (int64_t g = lane; g < n_groups; g += 32) {
+    const float e = box_distance2(mine, group[g]);
+    if (e < d) {
+      d = e;
+      at = g;
+    }
   }
-  if (i < n) out[i] = sqrtf(best);
+  const int64_t g0 = nearest(d, at);
+  {
+    const int64_t c = g0 * WD_C + lane;
+    const bool has = c < n_clusters;
+    visit(nearest(has ? box_distance2(mine, box[c]) : kWallFar, has ? c : g0 * WD_C));
+  }
+  for (int64_t gb = 0; gb < n_groups; gb += 32) {
+    const float eg = gb + lane < n_groups ? box_distance2(mine, group[gb + lane]) : kWallFar;
+    unsigned groups = __ballot_sync(0xffffffffu, gb + lane < n_groups && !(eg >= limit));
+    while (groups) {
+      const int gi = __ffs(groups) - 1;
+      groups &= groups - 1;
+      if (__shfl_sync(0xffffffffu, eg, gi) >= limit) continue;
+      const int64_t c = (gb + gi) * WD_C + lane;
+      const bool has = c < n_clusters;
+      const float ec = has ? box_distance2(mine, box[c]) : kWallFar;
+      unsigned clusters = __ballot_sync(0xffffffffu, has && !(ec >= limit));
+      while (clusters) {
+        const int ci = __ffs(clusters) - 1;
+        clusters &= clusters - 1;
+        if (__shfl_sync(0xffffffffu, ec, ci) >= limit) continue;
+        visit((gb + gi) * WD_C + ci);
+      }
+    }
+  }
+  if (in) out[i] = sqrtf(best);
 }
 
 }  // namespace mlp
@@ -1124,15 +1239,33 @@ int nf_mlp_predict(nf_mlp* m, const float* features, int64_t n, float* out, doub
 int nf_wall_distance(const float* points, int64_t n, const float* wall, int64_t m, float* out) {
   if (!points || !wall || !out || n <= 0 || m <= 0) return NF_ERR_ARG;
   try {
-    Buf<float> p, w, o;
-    p.alloc(size_t(3) * n);
-    w.alloc(size_t(3) * m);
-    o.alloc(size_t(n));
-    ck(cudaMemcpy(p.p, points, size_t(3) * n * sizeof(float), cudaMemcpyHostToDevice), "H2D");
-    ck(cudaMemcpy(w.p, wall, size_t(3) * m * sizeof(float), cudaMemcpyHostToDevice), "H2D");
-    wall_distance_kernel<<<unsigned((n + 255) / 256), 256>>>(p.p, n, w.p, m, o.p);
+    const int64_t n_clusters = (m + WD_C - 1) / WD_C, n_groups = (n_clusters + WD_C - 1) / WD_C;
+    // one allocation for all (each costs about 0.3 ms with its release)
+    Buf<float4> mem;
+    size_t used = 0;
+    auto place = [&used](size_t bytes) {
+      const size_t at = used;
+      used += (bytes + 255) / 256 * 256;
+      return at;
+    };
+    const size_t at_p = place(size_t(3) * n * sizeof(float)), at_w = place(size_t(3) * m * sizeof(float)),
+                 at_o = place(size_t(n) * sizeof(float)), at_wp = place(size_t(n_clusters) * WD_C * sizeof(float4)),
+                 at_box = place(size_t(n_clusters) * sizeof(WallBox)), at_group = place(size_t(n_groups) * sizeof(WallBox));
+    mem.alloc(used / sizeof(float4));
+    uint8_t* base = reinterpret_cast<uint8_t*>(mem.p);
+    float* p = reinterpret_cast<float*>(base + at_p);
+    float* w = reinterpret_cast<float*>(base + at_w);
+    float* o = reinterpret_cast<float*>(base + at_o);
+    float4* wp = reinterpret_cast<float4*>(base + at_wp);
+    WallBox* box = reinterpret_cast<WallBox*>(base + at_box);
+    WallBox* group = reinterpret_cast<WallBox*>(base + at_group);
+    ck(cudaMemcpy(p, points, size_t(3) * n * sizeof(float), cudaMemcpyHostToDevice), "H2D");
+    ck(cudaMemcpy(w, wall, size_t(3) * m * sizeof(float), cudaMemcpyHostToDevice), "H2D");
+    wall_cluster_kernel<<<unsigned((n_clusters + 7) / 8), 256>>>(w, m, n_clusters, wp, box);
+    wall_group_kernel<<<unsigned((n_groups + 7) / 8), 256>>>(box, n_clusters, n_groups, group);
+    wall_distance_kernel<<<unsigned((n + 255) / 256), 256>>>(p, n, wp, box, n_clusters, group, n_groups, o);
     ck(cudaGetLastError(), "wall distance launch");
-    ck(cudaMemcpy(out, o.p, size_t(n) * sizeof(float), cudaMemcpyDeviceToHost), "D2H");
+    ck(cudaMemcpy(out, o, size_t(n) * sizeof(float), cudaMemcpyDeviceToHost), "D2H");
   } catch (const std::exception& e) {
     g_mlp_error = e.what();
     return NF_ERR_CUDA;
