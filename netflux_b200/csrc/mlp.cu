@@ -933,7 +933,8 @@ std::string g_mlp_error;
 struct nf_mlp {
   cudaStream_t stream = nullptr;
   int n_sm = 148;
-  Buf<float> params, m, v, grad, partial, feat, target, out;
+  Buf<float> params, m, v, grad, partial, feat, target;
+  Buf<float> pred_in, pred_out;  // nf_mlp_predict's, kept (48 bytes a sample of the largest call)
   Buf<uint8_t> img_fwd, img_bwd;
   Buf<int> step;
   Buf<double> loss;
@@ -1206,7 +1207,7 @@ int nf_mlp_gradients(nf_mlp* m, const float* features, const float* targets, int
 int nf_mlp_predict(nf_mlp* m, const float* features, int64_t n, float* out, double* ms_out) {
   return mlp_guarded(m, [&]() -> int {
     if (!features || !out || n <= 0) return NF_ERR_ARG;
-    Buf<float> f, o;
+    Buf<float>&f = m->pred_in, &o = m->pred_out;
     f.alloc(size_t(n) * NIN);
     o.alloc(size_t(n) * NO);
     ck(cudaMemcpyAsync(f.p, features, size_t(n) * NIN * sizeof(float), cudaMemcpyHostToDevice, m->stream), "H2D");
