@@ -9,7 +9,8 @@
 //   2. a pair of variables at a time: limiter and face states of the tile's cells, and
 //      of each cut face's outside cell at that face, written over the pair's
 //      staged values once every thread has read them;
-//   3. boundary faces: ghost of the reconstructed state and its flux;
+//   3. boundary faces: ghost of the reconstructed state and its flux, each by the
+//      warp of its cell;
 //   4. per cell: four fluxes, the balance, the stage update;
 //   5. the ghosts of the result, for the next stage.
 // Nothing between the primitives and the updated state goes through HBM, and a
@@ -18,10 +19,10 @@
 // 160 B in, FP64) in four launches. The price is the limiter of the cut faces'
 // outside cells, 0.9 a cell at 256 cells a tile.
 //
-// A step, against those kernels: FP64 48,000 tets 62 -> 43 us, 153,600 tets (thin
-// tube) 95 -> 99 us, 3.1M tets 1.218 -> 1.128 ms; FP32 copies without
-// the limiter, 3.1M, 0.80 -> 0.76 ms; difference form 96,000 tets 74 -> 50 us, 393,216 183 -> 168 us, 3.1M
-// 1.051 -> 1.057 ms. Bound by latency: about 1,950 instructions a cell at 24
+// A step, against those kernels: FP64 48,000 tets 62 -> 42 us, 153,600 tets (thin
+// tube) 95 -> 98 us, 3.1M tets 1.218 -> 1.100 ms; FP32 copies without the limiter,
+// 3.1M, 0.80 -> 0.76 ms; difference form 96,000 tets 74 -> 49 us, 393,216 183 -> 159
+// us, 3.1M 1.051 -> 1.050 ms. Bound by latency: about 1,950 instructions a cell at 24
 // warps an SM (80 registers, three blocks), 38 % of issue slots and 29 % of the
 // FP64 pipe busy; of 13 cycles between a warp's instructions 4 wait for global
 // loads and 3 at barriers (393,216 tets, FP64). Loads of the tile that an SM
@@ -413,9 +414,28 @@ __global__ void __launch_bounds__(TC, kMinBlocks) stage_kernel(MeshView<double> 
   }
 
   // ---- 3. boundary faces: their fluxes after the face states, or (first order)
-  // in the place of their ghosts ----
+  // in the place of their ghosts. They lie in the order of their cells, so in second
+  // order a warp does those of its own cells, a range, and no other waits for it
+  // (a step of 48,000 tets 42.8 -> 41.6 us, of 393,216 in the difference form 168 ->
+  // 163 us, of 3.1M 1.118 -> 1.102 ms). In first order the block shares them: the
+  // kernel has little else to do (178,000 tets 1.1 % slower by warps) ----
+  [[maybe_unused]] int b_first = 1 << 30, b_end = 0;  // of this warp's cells (none: empty)
   if (h.nb > 0) {
-    for (int i = t; i < h.nb; i += TC) {
+    if constexpr (kSecond) {
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        if (code(q) >= n_states && code(q) != kFaceNone) {
+          b_first = min(b_first, code(q) - n_states);
+          b_end = max(b_end, code(q) - n_states + 1);
+        }
+      }
+      b_first = __reduce_min_sync(0xffffffffu, b_first);
+      b_end = __reduce_max_sync(0xffffffffu, b_end);
+    } else {
+      b_first = 0;
+      b_end = h.nb;
+    }
+    for (int i = b_first + (kSecond ? t & 31 : t); i < b_end; i += kSecond ? 32 : TC) {
       const int2 ref = tv.b_ref[h.b0 + i];
       const double4 geo = tv.b_geo[h.b0 + i];
       const int cb = checked(ref.x >> 2, m.n, a.status), q = ref.x & 3;
@@ -454,7 +474,8 @@ __global__ void __launch_bounds__(TC, kMinBlocks) stage_kernel(MeshView<double> 
         else rv[k * kRow + n1 + i] = V(S(fl.v[k]));
       }
     }
-    __syncthreads();
+    if constexpr (kSecond) __syncwarp();
+    else __syncthreads();
   }
 
   // ---- 4. fluxes and update ----
@@ -593,20 +614,17 @@ __global__ void __launch_bounds__(TC, kMinBlocks) stage_kernel(MeshView<double> 
   // ---- 5. the result's ghosts, which the next stage stages ----
   if constexpr (kMode == kModeGhosts || kGeneral) {
     if (h.nb > 0 && (kForm == kFormCopy ? a.vg_next32 != nullptr : a.vg_next != nullptr)) {
-      __syncthreads();  // the face states are no longer needed
-      if (act) {
-#pragma unroll
-        for (int k = 0; k < 5; k++) rv[k * kRow + t] = V(Vn[k]);
-      }
-      const bool live = __syncthreads_or(act);
-      for (int i = t; live && i < h.nb; i += TC) {
-        const int2 ref = tv.b_ref[h.b0 + i];
-        const int cb = checked(ref.x >> 2, m.n, a.status);
-        const int lc = checked(cb - int(blockIdx.x) * TC, TC, a.status);
-        if (frozen_cell(a, cb)) continue;  // keeps its state and its ghosts
+      for (int i0 = b_first; i0 < b_end; i0 += 32) {
+        const int i = i0 + (t & 31);
+        const bool mine = i < b_end;
+        int2 ref = make_int2(0, 0);
+        if (mine) ref = tv.b_ref[h.b0 + i];
+        const int src = checked(ref.x >> 2, m.n, a.status) & 31;  // its cell's lane
         FiveValues v;
 #pragma unroll
-        for (int k = 0; k < 5; k++) v.v[k] = double(rv[k * kRow + lc]);
+        for (int k = 0; k < 5; k++) v.v[k] = double(V(__shfl_sync(0xffffffffu, Vn[k], src)));
+        const bool moved = __shfl_sync(0xffffffffu, int(act), src) != 0;
+        if (!mine || !moved) continue;  // a converged case keeps its state and its ghosts
         const FiveValues g = boundary_ghost(m.patches + checked(ref.y, m.n_patches, a.status), tv.b_geo[h.b0 + i], v);
 #pragma unroll
         for (int k = 0; k < 5; k++) {
