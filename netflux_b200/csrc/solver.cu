@@ -382,9 +382,10 @@ struct nf_solver {
   // primitives are in place, and whatever else writes primitives clears it.
   // Up to kGhostWaves waves of tiles a kernel of its own (4 us a stage, mostly
   // launch) costs more than the boundary tiles' longer stay, beyond it less:
-  // a step of 48,000 tets 50 -> 46 us, of 393,216 (4 waves) 175 -> 174 us, of
-  // 3.1M (28 waves) 1.161 -> 1.167 ms.
-  static constexpr int kGhostWaves = 6;
+  // separate against left by the stage kernel, a step of 48,000 tets 45.8 -> 41.6 us,
+  // of 153,600 (1.4 waves) 100.3 -> 97.7, but of 393,216 (3.5 waves) 159 -> 163 and of
+  // 3.1M (28 waves) 1.100 -> 1.132 ms.
+  static constexpr int kGhostWaves = 2;
   bool own_ghosts() const { return n_tiles <= kGhostWaves * ahead && !copy_barth(); }  // the stage kernel leaves them
   bool ghosts_ready = false;
   double* vgbuf(int i) { return i && fast() ? vgb.p : vg.p; }
