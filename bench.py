@@ -15,7 +15,8 @@ Prints one JSON line on rank 0. ``value`` is Mcell-RK-stages/s with the state
 resident in HBM (CUDA events on the solver's stream, max over ranks);
 ``e2e`` is the same metric through the public API with the state copied
 host->device and back every step; ``roofline`` is the dominant kernel's
-algorithmic HBM bytes per launch over its event-timed duration against the
+algorithmic HBM bytes per launch (the fused stage kernel's, but for FP32
+copies under the Barth limiter) over its event-timed duration against the
 measured copy bandwidth; ``cpu_baseline`` is the NetFlux reference compiled
 from its sources, timed on this host's cores on a bounded sample.
 """
@@ -61,10 +62,11 @@ def parse():
                     help="skip timing the two mixed forms beside the FP64 step (FP64 runs only)")
     ap.add_argument("--steady-max", type=int, default=60000)
     ap.add_argument("--steady-limiter", choices=["none", "barth-ratchet"], default="none")
-    ap.add_argument("--block", type=int, default=0, help="fix the block size (no tuning)")
+    ap.add_argument("--block", type=int, default=0, help="fix the block size of the kernels that have one to choose (no tuning)")
     ap.add_argument("--variant", type=int, default=0, help="with --block: fast-kernel variant")
     ap.add_argument("--shapes", type=int, nargs=4, default=None, metavar=("GB", "GV", "FB", "FV"),
-                    help="fix the gradient and flux kernels' (block, variant) separately (no tuning)")
+                    help="fix the gradient and flux kernels' (block, variant) separately (no tuning); "
+                         "they run where the fused stage kernel does not: --precision mixed32")
     return ap.parse_args()
 
 
@@ -163,39 +165,46 @@ class ClockSampler:
                 "samples": len(sm)}
 
 
+def stage_bytes(n_cells: int, n_boundary: int, n_nodes: int, precision: str, local_dt: bool):
+    """Compulsory HBM bytes of one launch of the fused stage kernel (every datum it must read or
+    write, once; an outside cell's values are its own tile's and not counted again), averaged over
+    the three stages. Per cell:
+      own V (40; FP32 copies 20), face and vertex codes (8 + 8), the tile's lists of outside cells,
+      far cells and vertices (about 16), U (40), U^n (40 at stages 2 and 3), vol (8), local dt (8
+      with local time stepping), writes U and V (80; FP32 copies 60) and R_rho/vol at the first stage
+      (8), and once a step the next dt (reads the projected areas, 24; writes 8 with local time
+      stepping);
+    per node 32 (FP64) or 16 (FP32); per boundary face a ghost state (40; FP32 copies 20), unit
+    normal, area, owner and patch (40)."""
+    lts = 8 if local_dt else 0
+    f32 = precision == "mixed32"
+    cell = (20 if f32 else 40) + 16 + 16 + 40 + 40 * 2 / 3 + 8 + lts + (60 if f32 else 80) + (8 + 24 + lts) / 3
+    return n_cells * cell + n_nodes * (32 if precision == "fp64" else 16) + n_boundary * ((20 if f32 else 40) + 40)
+
+
 def algorithmic_bytes(n_cells: int, n_faces: int, n_boundary: int, n_nodes: int, precision: str,
                       local_dt: bool):
-    """Compulsory HBM bytes of one launch of each stage kernel (every datum the
-    kernel must read or write, once; neighbours' values are other cells' own
-    values and are not counted again), averaged over the three stages.
+    """Compulsory HBM bytes of one launch of each kernel where limiter and flux are kernels of their
+    own, which exchange four face states a cell (every datum read or written once, averaged over the
+    three stages). FP32 copies under the Barth limiter run that way; the FP64 and difference forms'
+    figures say what the fused kernel (stage_bytes) saves.
 
-    FP64 (gradient_node / flux_node), per cell:
-      gradient: V (40), 4 vertex ids (16), 4 neighbour ids (16), face code (4),
-        vol (8), writes 4 face states (160); per node 32 (xyz + pad); per
-        boundary face one ghost state (40); the last stage also writes the
-        next step's dt (8 with local time stepping; its projected areas come
-        from the normals in registers): a third of that on average.
-      flux: 4 own face states (160), 4 neighbour face ids (16), face code (4),
-        4 vertex ids (16), U (40), U^n (40 at stages 2 and 3: 2/3 on average),
-        vol (8), local dt (8 with local time stepping), writes U and V (80) and
-        R_rho/vol at the first stage (8, 1/3 on average); per node 32; per
-        boundary face one boundary flux (40).
-    Mixed (gradient_delta / flux_delta, FP32 differences to FP64 state):
-      gradient: V (40), ids (32), code (4), vol (8), writes 4 FP32 increments
-        (80); per node 16; per boundary face an FP64 ghost (40).
-      flux: own V (40), own increments (80), neighbour face ids (16), code (4),
-        vertex ids (16), U, U^n, vol, dt, writes U, V and R_rho as above; per
-        node 16; per boundary face an FP32 flux difference (20); stage 2 also
-        reads dS (24) and writes the next step's dt (8 with local time
-        stepping): a third of that on average.
-    Mixed with FP32 copies (the FP32 node kernels, NF_PREC_MIXED32):
-      gradient: FP32 V (20), ids (32), code (4), vol (8), writes 4 FP32 face
-        states (80); per node 16; per boundary face an FP32 ghost (20).
-      flux: 4 own FP32 face states (80), neighbour face ids (16), code (4),
-        vertex ids (16), U, U^n, vol, dt, writes U (40), the FP32 V (20) and
-        R_rho (no FP64 V: the stage-2 flux kernel computes the next dt from its
-        FP64 result); per node 16; per boundary face an FP32 flux (20); the
-        next step's dt as in the difference form.
+    FP64, per cell:
+      gradient: V (40), 4 vertex ids (16), 4 neighbour ids (16), face code (4), vol (8), writes 4
+        face states (160); per node 32 (xyz + pad); per boundary face one ghost state (40); the last
+        stage also writes the next step's dt (8 with local time stepping).
+      flux: 4 own face states (160), 4 neighbour face ids (16), face code (4), 4 vertex ids (16),
+        U (40), U^n (40 at stages 2 and 3: 2/3 on average), vol (8), local dt (8 with local time
+        stepping), writes U and V (80) and R_rho/vol at the first stage (8, 1/3 on average); per
+        node 32; per boundary face one boundary flux (40).
+    Mixed: FP32 increments (80) for the face states, FP64 V in both; stage 2 also reads dS (24) and
+      writes the next step's dt.
+    Mixed with FP32 copies (NF_PREC_MIXED32):
+      gradient: FP32 V (20), ids (32), code (4), vol (8), writes 4 FP32 face states (80); per node
+        16; per boundary face an FP32 ghost (20).
+      flux: 4 own FP32 face states (80), neighbour face ids (16), code (4), vertex ids (16), U, U^n,
+        vol, dt, writes U (40), the FP32 V (20) and R_rho; per node 16; per boundary face an FP32
+        flux (20); stage 2 also computes the next step's dt from its FP64 result.
     """
     lts = 8 if local_dt else 0
     upd = 40 + 40 * 2 / 3 + 8 + lts + 80 + 8 / 3  # U, U^n, vol, dt, U and V out, R_rho
@@ -212,16 +221,14 @@ def algorithmic_bytes(n_cells: int, n_faces: int, n_boundary: int, n_nodes: int,
     return {"flux": flux, "gradient": grad}
 
 
-# DRAM bytes per cell of one launch (dram__bytes_read.sum + dram__bytes_write.sum), captured
-# with ncu on the full 3,145,728-tet bump channel with the tuned launch shapes, averaged over the
-# three stages of a step like the event-timed launch durations (FP64: gradient 64/7, flux 64/9,
-# stages 755.3 / 749.8 / 780.6 and 1108.6 / 1221.7 / 1227.9 MB; mixed: gradient 64/7, flux
-# 128/8, stages 506.9 / 500.9 / 500.7 and 989.5 / 1208.8 / 1104.6 MB); the bump workload's
-# `roofline.traffic` is this times its cells, other workloads report null.
-MEASURED_DRAM_BYTES_PER_CELL = {
-    ("fp64", "gradient"): 761.9e6 / 3145728, ("fp64", "flux"): 1186.1e6 / 3145728,
-    ("mixed", "gradient"): 502.8e6 / 3145728, ("mixed", "flux"): 1101.0e6 / 3145728,
-}
+# DRAM bytes per cell of one launch of the fused stage kernel (dram__bytes_read.sum +
+# dram__bytes_write.sum), captured with ncu on the full 3,145,728-tet bump channel and averaged over
+# the three stages of a step (708.0 / 849.2 / 953.0 MB); the bump workload's `roofline.traffic` is this times its cells, other
+# workloads report null.
+STAGE_DRAM_BYTES_PER_CELL = {"fp64": 836.7e6 / 3145728}
+# The same of the separate limiter and flux kernels, by (precision, kernel): not captured for the
+# form that still runs them.
+MEASURED_DRAM_BYTES_PER_CELL = {}
 
 
 def model_bytes_per_cell_stage(n_cells: int, n_faces: int) -> float:
@@ -496,13 +503,20 @@ def main():
             ((L.NF_KERNEL_TIMESTEP, "timestep"), (L.NF_KERNEL_GRADIENT, "gradient"), (L.NF_KERNEL_FLUX, "flux"),
              (L.NF_KERNEL_OTHER, "other"))}
     nb = mesh.n_ghost
-    ab = algorithmic_bytes(N, mesh.n_faces, nb, int(mesh.info.n_nodes), args.precision, lts)
+    fused = kern["gradient"][1] == 0 and args.precision != "fp64_ref"
+    if fused:  # limiter, fluxes and update in one launch, booked as flux
+        ab = {"flux": stage_bytes(N, nb, int(mesh.info.n_nodes), args.precision, lts)}
+    else:
+        ab = algorithmic_bytes(N, mesh.n_faces, nb, int(mesh.info.n_nodes), args.precision, lts)
     hbm, hbm_kind = measured_peaks()
-    dom = max(("flux", "gradient"), key=lambda k: kern[k][0] * kern[k][1])
+    dom = max(ab, key=lambda k: kern[k][0] * kern[k][1])
     ach = ab[dom] / (kern[dom][0] * 1e-3) / 1e9
-    per_cell = MEASURED_DRAM_BYTES_PER_CELL.get((args.precision, dom)) if args.case == "bump" else None
+    per_cell = None
+    if args.case == "bump":
+        per_cell = (STAGE_DRAM_BYTES_PER_CELL.get(args.precision) if fused
+                    else MEASURED_DRAM_BYTES_PER_CELL.get((args.precision, dom)))
     traffic = int(per_cell * N) if per_cell else None
-    roof = {"bound": "hbm", "kernel": dom, "achieved": round(ach, 1), "peak": hbm, "unit": "GB/s",
+    roof = {"bound": "hbm", "kernel": "stage" if fused else dom, "achieved": round(ach, 1), "peak": hbm, "unit": "GB/s",
             "frac": round(ach / hbm, 4), "peak_kind": hbm_kind, "traffic": traffic,
             "algorithmic_bytes_per_launch": int(ab[dom]), "avg_launch_ms": round(kern[dom][0], 5),
             "per_kernel_ms": {k: round(v[0], 5) for k, v in kern.items()}}
@@ -620,7 +634,7 @@ def main():
             "config": {"workload": desc, "cells": N, "faces": mesh.n_faces, "time_scheme": "TVD_RK3",
                        "local_time_stepping": lts, "cfl": 0.8, "precision": args.precision,
                        "parallelism": f"replicas x{world}" if world > 1 else "single GPU",
-                       "l2": l2_note(model * N), "mesh_build_s": round(t_mesh, 2),
+                       "l2": l2_note(sum(ab.values())), "mesh_build_s": round(t_mesh, 2),
                        "launch_shapes": tuned},
             "roofline": roof,
             "step_roofline": {"model_bytes_per_cell_stage": round(model, 1), "achieved": round(step_gbs, 1),

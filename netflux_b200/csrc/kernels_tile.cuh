@@ -22,17 +22,18 @@
 // A step, against those kernels: FP64 48,000 tets 62 -> 42 us, 153,600 tets (thin
 // tube) 95 -> 98 us, 3.1M tets 1.218 -> 1.100 ms; FP32 copies without the limiter,
 // 3.1M, 0.80 -> 0.76 ms; difference form 96,000 tets 74 -> 49 us, 393,216 183 -> 159
-// us, 3.1M 1.051 -> 1.050 ms. Bound by latency: about 1,950 instructions a cell at 24
-// warps an SM (80 registers, three blocks), 38 % of issue slots and 29 % of the
-// FP64 pipe busy; of 13 cycles between a warp's instructions 4 wait for global
-// loads and 3 at barriers (393,216 tets, FP64). Loads of the tile that an SM
+// us, 3.1M 1.051 -> 1.050 ms. Bound by latency: about 1,860 instructions a cell at 24
+// warps an SM (80 registers, three blocks), 43 % of issue slots and 33 % of the
+// FP64 pipe busy; of 12.5 cycles between a warp's instructions 3 wait for global
+// loads and 2.6 at barriers (393,216 tets, FP64). Loads of the tile that an SM
 // takes a wave later are asked into L2 in bulk, which took 8 % off.
 //
 // Both cells of a face evaluate its flux from the same two states and opposite
 // normals of the same bits, with exactly antisymmetric arithmetic (rusanov_raw) or
-// with the owner on the left (FP32), and the outside cells' limiters are recomputed with the same operations on
-// the same values, so the two contributions cancel exactly, inside a tile or
-// across tiles, and a case gives the same bits alone or in a batch.
+// with the owner on the left (FP32), and the outside cells' limiters are recomputed
+// with the same operations on the same values, so the two contributions cancel
+// exactly, inside a tile or across tiles, and a case gives the same bits alone or
+// in a batch.
 #pragma once
 
 #include <type_traits>
