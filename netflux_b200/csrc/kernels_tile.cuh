@@ -47,8 +47,8 @@ enum : int { kFormFp64 = 0, kFormDelta = 1, kFormCopy = 2 };
 // what the stage kernel is compiled for: first order; second order, and the same
 // with the result's ghosts; or everything (the limiter ratchet, kept limiter
 // values, faces no marker lists, and the ghosts where asked for). At 3.1M tets the
-// FP64 launch takes 12 us more with the ghosts' code in it, unused, and 15 us more
-// with the ratchet's.
+// FP64 launch takes 17 us more when it leaves the ghosts (a kernel of their own 9.5
+// us), and took 15 us more with the ratchet's code in it, unused.
 enum : int { kModeFirst = 0, kModePlain = 1, kModeGhosts = 2, kModeGeneral = 3 };
 // staged primitives V, face states S (increments in the difference form) and
 // geometry G of each form
