@@ -30,6 +30,7 @@
 #include <algorithm>
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <random>
 #include <stdexcept>
 #include <string>
@@ -934,7 +935,11 @@ struct nf_mlp {
   cudaStream_t stream = nullptr;
   int n_sm = 148;
   Buf<float> params, m, v, grad, partial, feat, target;
-  Buf<float> pred_in, pred_out;  // nf_mlp_predict's, kept (48 bytes a sample of the largest call)
+  // nf_mlp_predict's, kept for calls of at most kPredictKept samples (200 MB); a
+  // call that finds them taken by another thread has buffers of its own
+  static constexpr int64_t kPredictKept = int64_t(1) << 22;
+  Buf<float> pred_in, pred_out;
+  std::mutex pred_mutex;
   Buf<uint8_t> img_fwd, img_bwd;
   Buf<int> step;
   Buf<double> loss;
@@ -1207,7 +1212,10 @@ int nf_mlp_gradients(nf_mlp* m, const float* features, const float* targets, int
 int nf_mlp_predict(nf_mlp* m, const float* features, int64_t n, float* out, double* ms_out) {
   return mlp_guarded(m, [&]() -> int {
     if (!features || !out || n <= 0) return NF_ERR_ARG;
-    Buf<float>&f = m->pred_in, &o = m->pred_out;
+    Buf<float> own_in, own_out;
+    std::unique_lock<std::mutex> lock(m->pred_mutex, std::defer_lock);
+    const bool kept = n <= nf_mlp::kPredictKept && lock.try_lock();
+    Buf<float>&f = kept ? m->pred_in : own_in, &o = kept ? m->pred_out : own_out;
     f.alloc(size_t(n) * NIN);
     o.alloc(size_t(n) * NO);
     ck(cudaMemcpyAsync(f.p, features, size_t(n) * NIN * sizeof(float), cudaMemcpyHostToDevice, m->stream), "H2D");
