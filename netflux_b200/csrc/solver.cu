@@ -470,10 +470,12 @@ struct nf_solver {
     prof_end();
   }
 
-  // primitives of U in both V buffers (as after nf_set_state)
+  // primitives of U in both V buffers (as after nf_set_state); a next time step
+  // computed from the ones before (zero in a converged case's cells) is not theirs
   void refresh_primitives() {
     for (int b = 0; b < 2; b++) launch_prim(U.p, b);
     ghosts_ready = false;
+    dt_ready = false;
   }
 
   void ratchet_reset() {
@@ -506,9 +508,11 @@ struct nf_solver {
     return std::min<int64_t>(n, p.limiter_ratchet_step - steps_done);
   }
 
-  // the captured steps take the ghosts as the step before left them
+  // the captured steps take the ghosts and the time step as the step before left
+  // them: one captured without would hold the kernels that compute them
   bool graph_ready() const {
-    return !fast() || p.spatial_order != NF_SECOND_ORDER || ghosts_ready || !own_ghosts();
+    return (!fast() || p.spatial_order != NF_SECOND_ORDER || ghosts_ready || !own_ghosts()) &&
+           (dt_stage() < 0 || dt_ready);
   }
 
   // n x (calc_timestep + step), replays of a two-step CUDA graph where
