@@ -694,13 +694,17 @@ __global__ void __launch_bounds__(128) gradient_field_kernel(MeshView<T> m, Stag
 // The next step's time step of one cell from the primitives the reference's
 // calc_timestep reads (a.dt_next_min set): written where local time stepping
 // keeps it; returns its part of the minimum. A frozen cell keeps its state (dt 0).
+// kRef: with the reference's operations and rounding, as timestep_kernel.
+template <bool kRef>
 __device__ __forceinline__ double cell_next_dt(const StageArgs& a, int c, int st, const double V[5], double vol,
                                                bool frozen) {
   if (frozen) {
     if (a.dt_next) a.dt_next[c] = 0.0;
     return DBL_MAX;
   }
-  const double d = dt_of_cell_fast(V, a.dS[c], a.dS[st + c], a.dS[2 * st + c], vol, a.cfl);
+  double d;
+  if constexpr (kRef) d = dt_of_cell(V, a.dS[c], a.dS[st + c], a.dS[2 * st + c], vol, a.cfl);
+  else d = dt_of_cell_fast(V, a.dS[c], a.dS[st + c], a.dS[2 * st + c], vol, a.cfl);
   if (a.dt_next) a.dt_next[c] = d;
   if (!(d > 0.0) && !isnan(d)) atomicOr(a.status, kErrDt);
   return d > 0.0 ? d : DBL_MAX;  // std::min skips NaN (comparisons with NaN are false)
@@ -758,7 +762,7 @@ __device__ __forceinline__ double stage_update(const StageArgs& a, int c, int st
   if (a.res_cell) a.res_cell[c] = R[0] * ivol;
   if (top >= 0x7ff00000) atomicOr(a.status, kErrNonFinite);
   else if (!(Vn[0] > 0.0) || !(Vn[4] > 0.0)) atomicOr(a.status, kErrNonPhysical);
-  return a.dt_next_min && !a.dt_from_input ? cell_next_dt(a, c, st, Vn, vol, a.freeze && dt == 0.0) : DBL_MAX;
+  return a.dt_next_min && !a.dt_from_input ? cell_next_dt<false>(a, c, st, Vn, vol, a.freeze && dt == 0.0) : DBL_MAX;
 }
 
 // ---------------------------------------------------------------------------

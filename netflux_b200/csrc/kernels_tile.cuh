@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(TC, kMinBlocks) stage_kernel(MeshView<double> 
     for (int k = 0; k < 5; k++) rv[k * kRow + t] = own[k];
     if constexpr (kForm != kFormCopy) {
       if (a.dt_from_input) {
-        const double d = in ? cell_next_dt(a, c, st, own, m.vol[c], !act) : DBL_MAX;
+        const double d = in ? cell_next_dt<kForm == kFormFp64 && !kSecond>(a, c, st, own, m.vol[c], !act) : DBL_MAX;
         warp_min_to(d, a.dt_next_min);
       }
     }

@@ -410,9 +410,16 @@ struct nf_solver {
   // from its result; -1: none (timestep_kernel does)
   int dt_stage() const {
     if (!fast() || p.dt_from_current_state) return -1;
-    if (p.precision != NF_PREC_MIXED32) return n_stages() - 1;
-    return p.time_scheme == NF_TVD_RK3 ? n_stages() - 2 : -1;
+    if (p.precision == NF_PREC_FP64) return n_stages() - 1;
+    if (p.time_scheme != NF_TVD_RK3) return -1;
+    return p.precision == NF_PREC_MIXED ? n_stages() - 1 : n_stages() - 2;
   }
+  // FP64 first order: only where the same call takes the next step too. Between
+  // calls the step's own dt stays in place, for the steps and getters that follow
+  // without a nf_calc_timestep, and the next one is timestep_kernel's; the stage
+  // kernel rounds as that kernel does. Twenty steps of 178,000 tets, state in and
+  // out, take 1.641 ms so, the same as with every next time step computed ahead.
+  bool dt_within_call() const { return p.precision == NF_PREC_FP64 && p.spatial_order != NF_SECOND_ORDER; }
   // primitives of Usrc into primitive buffer b (and its FP32 copy in the
   // mixed form with FP32 copies)
   void launch_prim(const double* Usrc, int b) {
@@ -457,6 +464,7 @@ struct nf_solver {
     scal_kernel<<<1, 1, 0, stream>>>(scal.p, 0, status.p);
     prof_end();
     nf::DtArgs a;
+    if (dt_stage() >= 0) dtl_cur = vcur;  // the dt buffer that the graph of this vcur holds
     const int vb = p.dt_from_current_state ? vcur : (stepped ? 1 - vcur : vcur);
     a.V = Vbuf(vb);
     a.cfl = p.cfl;
@@ -515,13 +523,20 @@ struct nf_solver {
            (dt_stage() < 0 || dt_ready);
   }
 
+  // two of the next `left` steps by a graph, `rest` more steps of this call after
+  // them (the graphs' steps compute the next time step: never the call's last one
+  // where that must not, dt_within_call)
+  bool graph_next(int64_t left, int64_t rest) const {
+    return left >= 2 && stepped && graph_ready() && (left + rest > 2 || !dt_within_call());
+  }
+
   // n x (calc_timestep + step), replays of a two-step CUDA graph where
   // possible; the ratchet starts at its step.
   void run_steps(int64_t n) {
     if (n > 0 && old_pending) {  // this step's U^n is not U: outside the graphs
       ratchet_due(1);
       enqueue_dt();
-      enqueue_step();
+      enqueue_step(n > 1);
       steps_done++;
       n--;
     }
@@ -529,7 +544,7 @@ struct nf_solver {
       int64_t left = ratchet_due(n);
       n -= left;
       steps_done += left;
-      if (left >= 2 && stepped && graph_ready()) {
+      if (graph_next(left, n)) {
         const int v0 = vcur;
         if (!graph[v0]) {
           // capture two steps: the V buffers return to their roles afterwards
@@ -537,24 +552,24 @@ struct nf_solver {
           ck(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "begin capture");
           for (int k = 0; k < 2; k++) {
             enqueue_dt();
-            enqueue_step();
+            enqueue_step(true);
           }
           ck(cudaStreamEndCapture(stream, &g), "end capture");
           ck(cudaGraphInstantiate(&graph[v0], g, 0), "graph instantiate");
           cudaGraphDestroy(g);
           vcur = v0;
         }
-        while (left >= 2) {
+        while (graph_next(left, n)) {
           ck(cudaGraphLaunch(graph[v0], stream), "graph launch");
           left -= 2;
         }
       }
       while (left > 0) {
         enqueue_dt();
-        enqueue_step();
+        enqueue_step(left + n > 1);
         left--;
         // the rest by graph, where there is one or its capture (about 0.2 ms) pays
-        if (left >= (graph[vcur] ? 2 : 32) && graph_ready()) break;
+        if ((graph[vcur] || left >= 32) && graph_next(left, n)) break;
       }
       n += left;
       steps_done -= left;
@@ -658,15 +673,16 @@ struct nf_solver {
   int n_stages() const { return p.time_scheme == NF_TVD_RK3 ? 3 : 1; }
   int stage_next = 0;  // the next stage nf_stage may enqueue
 
-  void enqueue_step() {
-    for (int s = 0; s < n_stages(); s++) enqueue_stage(s);
+  // more: this call takes another step after it
+  void enqueue_step(bool more) {
+    for (int s = 0; s < n_stages(); s++) enqueue_stage(s, more);
     stage_next = 0;
   }
 
   // One stage of the step; the last one also ends the step.
-  void enqueue_stage(int s) {
+  void enqueue_stage(int s, bool more) {
     const int n_stages = this->n_stages();
-    const bool fuse = dt_stage() >= 0;
+    const bool fuse = dt_stage() >= 0 && (more || !dt_within_call());
     {
       nf::StageArgs a{};
       a.second_order = p.spatial_order == NF_SECOND_ORDER;
@@ -784,10 +800,8 @@ struct nf_solver {
     prof_begin(NF_KERNEL_OTHER);
     scal_kernel<<<1, 1, 0, stream>>>(scal.p, fuse ? 2 : 1, status.p);
     prof_end();
-    if (fuse) {
-      dtl_cur = 1 - dtl_cur;
-      dt_ready = true;
-    }
+    if (fuse) dtl_cur = 1 - dtl_cur;
+    dt_ready = fuse;
     stepped = true;
     old_pending = false;  // solution_old = solution (Solver.cpp:51)
   }
@@ -953,7 +967,7 @@ struct nf_split {
       ck(cudaStreamWaitEvent(parts[i]->stream, dt_done, 0), "cudaStreamWaitEvent");
     }
   }
-  void step() {
+  void step(bool more) {
     for (nf_solver* s : parts) {
       set_dev(s->device);
       s->ratchet_due(1);
@@ -965,7 +979,7 @@ struct nf_split {
       exchange(k);
       for (nf_solver* s : parts) {
         set_dev(s->device);
-        s->enqueue_stage(k);
+        s->enqueue_stage(k, more);
       }
     }
     for (nf_solver* s : parts) s->steps_done++;
@@ -1764,7 +1778,7 @@ int nf_step(nf_solver* s) {
       return NF_ERR_ARG;
     }
     s->ratchet_due(1);
-    s->enqueue_step();
+    s->enqueue_step(false);
     s->steps_done++;
     ck(cudaGetLastError(), "step launch");
     return NF_OK;
@@ -1779,7 +1793,7 @@ int nf_stage(nf_solver* s, int stage) {
       return NF_ERR_ARG;
     }
     if (stage == 0) s->ratchet_due(1);
-    s->enqueue_stage(stage);
+    s->enqueue_stage(stage, false);
     s->stage_next = (stage + 1) % s->n_stages();
     if (s->stage_next == 0) s->steps_done++;
     ck(cudaGetLastError(), "stage launch");
@@ -2061,14 +2075,23 @@ int nf_time_steps(nf_solver* s, int64_t n_steps, int per_kernel, double* ms_tota
     }
     ck(cudaEventRecord(e0, s->stream), "cudaEventRecord");
     int64_t left = n_steps;
-    if (!per_kernel && left >= 2 && s->stepped && s->graph_ready()) {
+    float ms_first = 0.f;  // of a step before the graph was captured
+    if (!per_kernel && left > 2 && s->stepped && !s->graph_ready()) {  // a step that leaves what the graphs take
+      s->enqueue_dt();
+      s->enqueue_step(true);
+      left--;
+    }
+    if (!per_kernel && s->graph_next(left, 0)) {
       const int v0 = s->vcur;
       if (!s->graph[v0]) {
+        ck(cudaEventRecord(e1, s->stream), "cudaEventRecord");
+        ck(cudaEventSynchronize(e1), "cudaEventSynchronize");
+        ck(cudaEventElapsedTime(&ms_first, e0, e1), "cudaEventElapsedTime");
         cudaGraph_t g = nullptr;
         ck(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
         for (int k = 0; k < 2; k++) {
           s->enqueue_dt();
-          s->enqueue_step();
+          s->enqueue_step(true);
         }
         ck(cudaStreamEndCapture(s->stream, &g), "end capture");
         ck(cudaGraphInstantiate(&s->graph[v0], g, 0), "graph instantiate");
@@ -2081,14 +2104,14 @@ int nf_time_steps(nf_solver* s, int64_t n_steps, int per_kernel, double* ms_tota
         ck(cudaStreamSynchronize(s->stream), "cudaStreamSynchronize");
         ck(cudaEventRecord(e0, s->stream), "cudaEventRecord");
       }
-      while (left >= 2) {
+      while (s->graph_next(left, 0)) {
         ck(cudaGraphLaunch(s->graph[v0], s->stream), "graph launch");
         left -= 2;
       }
     }
     while (left > 0) {
       s->enqueue_dt();
-      s->enqueue_step();
+      s->enqueue_step(left > 1);
       left--;
     }
     s->steps_done += n_steps;  // timing runs count as steps but do not start the ratchet
@@ -2096,7 +2119,7 @@ int nf_time_steps(nf_solver* s, int64_t n_steps, int per_kernel, double* ms_tota
     ck(cudaEventSynchronize(e1), "cudaEventSynchronize");
     float ms = 0.f;
     ck(cudaEventElapsedTime(&ms, e0, e1), "cudaEventElapsedTime");
-    *ms_total = ms;
+    *ms_total = ms + ms_first;
     if (per_kernel) {
       s->prof_on = false;
       if (kernel_ms)
@@ -2291,7 +2314,7 @@ int nf_split_advance(nf_split* sp, int64_t n_steps) {
         sp->err = "nf_split_advance: a part is inside a step";
         return NF_ERR_ARG;
       }
-    for (int64_t k = 0; k < n_steps; k++) sp->step();
+    for (int64_t k = 0; k < n_steps; k++) sp->step(k + 1 < n_steps);
     return NF_OK;
   });
 }
