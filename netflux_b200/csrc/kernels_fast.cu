@@ -154,10 +154,11 @@ void launch_gradient_field(int form, const MeshView<double>& m, const MeshView<f
 
 // The cell-centre ghost state of every boundary face from the stage input's
 // primitives (set_constant_ghost_values, Solver.cpp:300-330), where the previous
-// stage kernel did not leave it. kCopy: from the FP32 primitives, computed in
-// FP64 (boundary faces are a few percent of the faces), stored in FP32, with the
-// powers as ever (kernels_copy.cuh says why).
-template <bool kCopy>
+// stage kernel did not leave it, by the function the stage kernel calls, so that it
+// is the same state wherever it is computed. kCopy: from the FP32 primitives,
+// computed in FP64 (boundary faces are a few percent of the faces), stored in FP32.
+// kPowers: for the kernels of kernels_copy.cuh, with the powers as ever.
+template <bool kCopy, bool kPowers>
 __global__ void __launch_bounds__(256) ghost_kernel_fast(MeshView<double> m, TileView tv, StageArgs a) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   pdl_launch_dependents();
@@ -166,20 +167,27 @@ __global__ void __launch_bounds__(256) ghost_kernel_fast(MeshView<double> m, Til
   const int2 ref = tv.b_ref[b];
   const double4 geo = tv.b_geo[b];
   const int c = checked(ref.x >> 2, m.n, a.status), st = m.stride;
-  const double nh[3] = {geo.x, geo.y, geo.z};
-  double V[5], G[5];
+  const PatchBC* bc = m.patches + checked(ref.y, m.n_patches, a.status);
+  FiveValues V, G;
 #pragma unroll
-  for (int k = 0; k < 5; k++) V[k] = kCopy ? double(a.Vin32[k * st + c]) : a.Vin[k * st + c];
-  ghost_state<double, kCopy>(m.patches[checked(ref.y, m.n_patches, a.status)], V, nh, G);
+  for (int k = 0; k < 5; k++) V.v[k] = kCopy ? double(a.Vin32[k * st + c]) : a.Vin[k * st + c];
+  if constexpr (kPowers) {
+    const double nh[3] = {geo.x, geo.y, geo.z};
+    ghost_state<double, true>(*bc, V.v, nh, G.v);
+  } else {
+    G = boundary_ghost(bc, geo, V);
+  }
 #pragma unroll
   for (int k = 0; k < 5; k++) {
-    if constexpr (kCopy) a.vg32[k * m.bstride + b] = float(G[k]);
-    else a.vg[k * m.bstride + b] = G[k];
+    if constexpr (kCopy) a.vg32[k * m.bstride + b] = float(G.v[k]);
+    else a.vg[k * m.bstride + b] = G.v[k];
   }
 }
-void launch_ghost(int form, const MeshView<double>& m, const TileView& tv, const StageArgs& a, Launch l) {
+void launch_ghost(int form, bool powers, const MeshView<double>& m, const TileView& tv, const StageArgs& a, Launch l) {
   if (m.nb == 0) return;
-  auto* k = form == kFormCopy ? ghost_kernel_fast<true> : ghost_kernel_fast<false>;
+  auto* k = form != kFormCopy ? ghost_kernel_fast<false, false>
+            : powers          ? ghost_kernel_fast<true, true>
+                              : ghost_kernel_fast<true, false>;
   launch_pdl(k, grid_for(m.nb, l.block), l.block, 0, l.stream, m, tv, a);
 }
 __global__ void fastmath_kernel(const double* x, int n, double* rcp, double* rsq) {

@@ -38,8 +38,9 @@ void launch_bflux_copy(const MeshView<double>& m, const TileView& tv, const Stag
 // the gradient field of a stage's input (keep_stage_fields)
 void launch_gradient_field(int form, const MeshView<double>& m, const MeshView<float>& m32, const StageArgs& a,
                            cudaStream_t st);
-// cell-centre ghost states of the stage's input, FP64 or (FP32 copies) FP32
-void launch_ghost(int form, const MeshView<double>& m, const TileView& tv, const StageArgs& a, Launch l);
+// cell-centre ghost states of the stage's input, FP64 or (FP32 copies) FP32;
+// powers: the far field's by pow (FP32 copies under the Barth limiter)
+void launch_ghost(int form, bool powers, const MeshView<double>& m, const TileView& tv, const StageArgs& a, Launch l);
 void launch_prim_fast(int n, int stride, const double* U, double* V, float* V32, Launch l);
 // the fast forms' reciprocal and reciprocal square root, elementwise (self-test)
 void launch_fastmath(const double* x, int n, double* rcp, double* rsq, Launch l);

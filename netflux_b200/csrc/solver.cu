@@ -578,7 +578,7 @@ struct nf_solver {
 
   void launch_ghost(const nf::StageArgs& a) {
     if (p.precision == NF_PREC_FP64_REF) nf::launch_ghost_ref(view64(), a, launch());
-    else nf::launch_ghost(form(), view64(), tiles(), a, launch());
+    else nf::launch_ghost(form(), copy_barth(), view64(), tiles(), a, launch());
   }
   // launch variants accepted by nf_set_launch_shapes (gradient, flux)
   int grad_variants() const { return 10; }
