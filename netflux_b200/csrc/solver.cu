@@ -49,9 +49,12 @@ struct DevBuf {
     n = count;
     if (count) ck(cudaMalloc(&p, count * sizeof(T)), "cudaMalloc");
   }
+  // returns when h has been read: the caller may free or change it
   void upload(const std::vector<T>& h, cudaStream_t s) {
     alloc(h.size());
-    if (n) ck(cudaMemcpyAsync(p, h.data(), n * sizeof(T), cudaMemcpyHostToDevice, s), "cudaMemcpyAsync H2D");
+    if (!n) return;
+    ck(cudaMemcpyAsync(p, h.data(), n * sizeof(T), cudaMemcpyHostToDevice, s), "cudaMemcpyAsync H2D");
+    ck(cudaStreamSynchronize(s), "cudaStreamSynchronize");
   }
   void zero(cudaStream_t s) {
     if (n) ck(cudaMemsetAsync(p, 0, n * sizeof(T), s), "cudaMemsetAsync");
@@ -1291,7 +1294,6 @@ nf_solver* nf_create(const nf_mesh* h, const nf_params* params) {
       s->b_slot.upload(hb_slot, st);
       s->b_face.upload(hb_face, st);
       s->b_patch.upload(hb_patch, st);
-      ck(cudaStreamSynchronize(st), "cudaStreamSynchronize");  // the host arrays end here
     }
     // node-based layout of the fast forms: a cell's vertices sorted by node
     // id; face m is the face opposite vertex m
