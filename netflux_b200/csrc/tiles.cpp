@@ -6,6 +6,7 @@
 #include <exception>
 #include <mutex>
 #include <stdexcept>
+#include <system_error>
 #include <thread>
 #include <utility>
 
@@ -188,7 +189,14 @@ Tiles build_tiles(int n, int stride, int tile, const std::vector<int>& nbvf, con
     }
   };
   std::vector<std::thread> pool;
-  for (int w = 1; w < n_threads; w++) pool.emplace_back(guarded, w);
+  pool.reserve(size_t(n_threads));
+  for (int w = 1; w < n_threads; w++) {
+    try {
+      pool.emplace_back(guarded, w);
+    } catch (const std::system_error&) {  // no further thread: its range by this one
+      guarded(w);
+    }
+  }
   guarded(0);
   for (auto& th : pool) th.join();
   if (failed) std::rethrow_exception(failed);
