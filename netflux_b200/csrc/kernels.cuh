@@ -73,7 +73,8 @@ struct MeshView {
 };
 
 // Index checks of NF_DEBUG builds (make debug): every index a kernel reads
-// from the mesh arrays is checked before it is used; an index out of range
+// from the mesh arrays or a tile's lists is checked before it is used (the lists'
+// own bounds, TileHead, are not); an index out of range
 // sets kErrIndex in the status word and is replaced by a valid one (0, or the
 // cell itself), so the access stays in bounds and the host reports the error.
 // In the release build these are the identity.

@@ -212,7 +212,16 @@ __global__ void __launch_bounds__(TC, kMinBlocks) stage_kernel(MeshView<double> 
 #pragma unroll
     for (int e = 0; e < 3; e++) nodes[3 * i + e] = p[e];
   }
+  // two spellings: the checked one, though checked() is the identity in the release
+  // build, made first order 4 % slower there (745 against 716 us a step of 3.1M tets)
+#ifdef NF_DEBUG
+  auto code = [&](int q) {
+    const int v = int(((q & 2) ? code4.y : code4.x) >> (16 * (q & 1)) & 0xffffu);
+    return v == kFaceNone ? v : checked(v, 4 * TC + h.ncut + h.nb, a.status);
+  };
+#else
   auto code = [&](int q) { return int(((q & 2) ? code4.y : code4.x) >> (16 * (q & 1)) & 0xffffu); };
+#endif
   auto vert = [&](int q) { return int(((q & 2) ? vert4.y : vert4.x) >> (16 * (q & 1)) & 0xffffu); };
   pdl_wait_previous();
   const bool act = in && !(a.case_frozen != nullptr && a.case_frozen[h.case_id >= 0 ? h.case_id : a.cell_case[c]] != 0);
@@ -358,7 +367,9 @@ __global__ void __launch_bounds__(TC, kMinBlocks) stage_kernel(MeshView<double> 
         const int i = r * TC + t;
         if (r * TC < h.ncut && i < h.ncut) {
           const int slot = cn[r].x >> 14;
-          const int nc[4] = {cn[r].x & 0x3fff, cn[r].y, cn[r].z, cn[r].w};
+          const int n_staged = n2 + h.nfar;
+          const int nc[4] = {checked(cn[r].x & 0x3fff, n_staged, a.status), checked(cn[r].y, n_staged, a.status),
+                             checked(cn[r].z, n_staged, a.status), checked(cn[r].w, n_staged, a.status)};
           unsigned nn = 0;
           if constexpr (!kLean) {
 #pragma unroll
@@ -488,7 +499,7 @@ __global__ void __launch_bounds__(TC, kMinBlocks) stage_kernel(MeshView<double> 
 #pragma unroll
     for (int q = 0; q < 4; q++)
 #pragma unroll
-      for (int e = 0; e < 3; e++) P[q][e] = nodes[3 * (vert(q) & kVertIndex) + e];
+      for (int e = 0; e < 3; e++) P[q][e] = nodes[3 * checked(vert(q) & kVertIndex, h.nnode, a.status) + e];
     // a boundary face's flux, or nothing for a face not listed; true: an interior face
     using Acc = typename std::conditional<kForm == kFormDelta, double, S>::type;
     Acc R[5] = {Acc(0), Acc(0), Acc(0), Acc(0), Acc(0)};
