@@ -223,12 +223,16 @@ def algorithmic_bytes(n_cells: int, n_faces: int, n_boundary: int, n_nodes: int,
 
 # DRAM bytes per cell of one launch of the fused stage kernel (dram__bytes_read.sum +
 # dram__bytes_write.sum), captured with ncu on the full 3,145,728-tet bump channel and averaged over
-# the three stages of a step (708.0 / 849.2 / 953.0 MB); the bump workload's `roofline.traffic` is this times its cells, other
-# workloads report null.
-STAGE_DRAM_BYTES_PER_CELL = {"fp64": 836.7e6 / 3145728}
-# The same of the separate limiter and flux kernels, by (precision, kernel): not captured for the
-# form that still runs them.
-MEASURED_DRAM_BYTES_PER_CELL = {}
+# the three stages of a step (FP64 708.0 / 849.2 / 953.0 MB, differences 686.9 / 815.6 / 912.9 MB);
+# the bump workload's `roofline.traffic` is this times its cells, other workloads report null.
+STAGE_DRAM_BYTES_PER_CELL = {"fp64": 836.7e6 / 3145728, "mixed": 805.1e6 / 3145728}
+# The same of the separate limiter and flux kernels, by (precision, kernel), for the form that runs
+# them (FP32 copies, shapes 64 9 128 9; stages 426.4 / 427.1 / 426.2 and 751.2 / 957.5 / 856.5 MB).
+MEASURED_DRAM_BYTES_PER_CELL = {("mixed32", "gradient"): 426.6e6 / 3145728,
+                                ("mixed32", "flux"): 855.0e6 / 3145728}
+# Forms whose kernels come in several launch shapes (nf_tune times them); the others' stage kernel
+# has the one that its mesh calls for, and their lines carry no shapes.
+FORMS_WITH_SHAPES = ("mixed32",)
 
 
 def model_bytes_per_cell_stage(n_cells: int, n_faces: int) -> float:
@@ -379,7 +383,7 @@ def mixed_forms(mesh, cfg_kw: dict, U0, steps: int, warmup: int, fp64_ms: float,
         cfg = S.Config(precision=prec, **cfg_kw)
         s = S.EulerSolver(cfg, mesh, U0=U0, device=device)
         s.advance(max(warmup, 3) - 2)
-        shapes = s.tune()
+        shapes = s.tune() if prec in FORMS_WITH_SHAPES else None
         s.advance(2)
         ms = C.c_double()
         kms = (C.c_double * L.NF_KERNEL_COUNT)()
@@ -471,7 +475,9 @@ def main():
     if args.shapes:  # fixed before the warm-up, so every launch has these shapes
         solver.set_launch_shapes(gradient=args.shapes[:2], flux=args.shapes[2:])
     solver.advance(max(args.warmup, 3) - 2)
-    if args.shapes:
+    if args.precision not in FORMS_WITH_SHAPES:
+        tuned = None
+    elif args.shapes:
         tuned = {"gradient": {"block": args.shapes[0], "variant": args.shapes[1]},
                  "flux": {"block": args.shapes[2], "variant": args.shapes[3]}, "fixed": True}
     else:
