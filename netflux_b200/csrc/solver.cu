@@ -265,7 +265,7 @@ struct nf_solver {
 
   // mesh
   DevBuf<int> slot, nbslot, b_cell, b_slot, b_face, b_patch;  // boundary faces of the reference-order form
-  DevBuf<int> cnode, gcode, nbvf, nbsf;  // node-based layout of the fast forms (nbsf: copy_barth)
+  DevBuf<int> cnode, gcode, nbvf, nbsf;  // node-based layout (copy_barth; without nbsf, kept stage fields)
   DevBuf<double> S, nhat, area, rs, vol, dS, nodes4;
   DevBuf<float> nodes4_32;
   // tiles of the fast forms' stage kernel
@@ -1399,9 +1399,11 @@ nf_solver* nf_create(const nf_mesh* h, const nf_params* params) {
     }
 
     if (fast) {
-      s->gcode.upload(h_gcode, st);
-      s->cnode.upload(h_cnode, st);
-      s->nbvf.upload(h_nbvf, st);
+      if (s->copy_barth() || p.keep_stage_fields) {  // what the stage kernel does not read
+        s->gcode.upload(h_gcode, st);
+        s->cnode.upload(h_cnode, st);
+        s->nbvf.upload(h_nbvf, st);
+      }
       if (!s->copy_barth()) {
         int max_smem = 0;
         ck(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device), "attr");
