@@ -216,8 +216,7 @@ __device__ __forceinline__ double stage_dt(const double* scal) {
   return dt;
 }
 
-// The templated kernels below run in FP64 (T = double); the mixed form has
-// its own kernels (kernels_mixed.cuh).
+// The reference-order kernels run in FP64 (T = double).
 template <typename T>
 __device__ __forceinline__ T ld_v(const StageArgs& a, int idx) {
   static_assert(sizeof(T) == 8, "FP64 kernels");
@@ -237,33 +236,6 @@ __device__ __forceinline__ T quad_sum_ordered(T v) {
   for (int p = 0; p < 4; p++) s = s + __shfl_sync(kFull, v, p, 4);
   return s;
 }
-template <typename T>
-__device__ __forceinline__ T quad_max_ordered(T init, T v) {
-#pragma unroll
-  for (int p = 0; p < 4; p++) init = rmax(init, __shfl_sync(kFull, v, p, 4));
-  return init;
-}
-template <typename T>
-__device__ __forceinline__ T quad_min_ordered(T init, T v) {
-#pragma unroll
-  for (int p = 0; p < 4; p++) init = rmin(init, __shfl_sync(kFull, v, p, 4));
-  return init;
-}
-template <typename T>
-__device__ __forceinline__ T quad_sum_tree(T v) {
-  v = v + __shfl_xor_sync(kFull, v, 1, 4);
-  return v + __shfl_xor_sync(kFull, v, 2, 4);
-}
-template <typename T>
-__device__ __forceinline__ T quad_min_tree(T v) {
-  v = fmin(v, __shfl_xor_sync(kFull, v, 1, 4));
-  return fmin(v, __shfl_xor_sync(kFull, v, 2, 4));
-}
-template <typename T>
-__device__ __forceinline__ T quad_max_tree(T v) {
-  v = fmax(v, __shfl_xor_sync(kFull, v, 1, 4));
-  return fmax(v, __shfl_xor_sync(kFull, v, 2, 4));
-}
 
 // ---------------------------------------------------------------------------
 // Green-Gauss gradient + min/max + Barth limiter
@@ -279,7 +251,7 @@ __device__ __forceinline__ T quad_max_tree(T v) {
 // folds its cell's faces in slot order, exactly as the reference's face loops
 // reach that cell.
 // ---------------------------------------------------------------------------
-template <typename T, bool kRef>
+template <typename T>
 __global__ void __launch_bounds__(256) gradient_limiter_kernel(MeshView<T> m, StageArgs a) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int c = t / 5;
@@ -312,26 +284,10 @@ __global__ void __launch_bounds__(256) gradient_limiter_kernel(MeshView<T> m, St
     const T Sg[3] = {own ? s0 : -s0, own ? s1 : -s1, own ? s2 : -s2};
     const T uf = T(0.5) * (vc + vo);  // 0.5 (V_i + V_j); the sum commutes exactly
 #pragma unroll
-    for (int d = 0; d < 3; d++) {
-      if constexpr (kRef) g[d] = g[d] + uf * Sg[d] / vol;
-      else g[d] = fma(uf, Sg[d], g[d]);
-    }
-    if constexpr (kRef) {
-      const T vi = own ? vc : vo, vj = own ? vo : vc;  // max(V_i, V_j) in the face's operand order
-      vmax = rmax(vmax, rmax(vi, vj));
-      vmin = rmin(vmin, rmin(vi, vj));
-    } else {
-      vmax = fmax(vmax, vo);
-      vmin = fmin(vmin, vo);
-    }
-  }
-  if constexpr (!kRef) {
-    const T iv = T(1) / vol;
-    g[0] *= iv;
-    g[1] *= iv;
-    g[2] *= iv;
-    vmax = fmax(vmax, vc);
-    vmin = fmin(vmin, vc);
+    for (int d = 0; d < 3; d++) g[d] = g[d] + uf * Sg[d] / vol;
+    const T vi = own ? vc : vo, vj = own ? vo : vc;  // max(V_i, V_j) in the face's operand order
+    vmax = rmax(vmax, rmax(vi, vj));
+    vmin = rmin(vmin, rmin(vi, vj));
   }
   // grad V_k . r at each face: the limiter's Delta_2 before its sign/epsilon
   // adjustment, and the increment of the reconstruction
@@ -379,7 +335,7 @@ __global__ void __launch_bounds__(256) gradient_limiter_kernel(MeshView<T> m, St
 // The face states come from gradient_limiter_kernel (second order) or are the
 // cell primitives (first order). Lane q evaluates the flux of face slot q.
 // ---------------------------------------------------------------------------
-template <typename T, bool kRef>
+template <typename T>
 __global__ void __launch_bounds__(256) flux_update_kernel(MeshView<T> m, StageArgs a) {
   const int q = threadIdx.x & 3;
   int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
@@ -418,25 +374,17 @@ __global__ void __launch_bounds__(256) flux_update_kernel(MeshView<T> m, StageAr
     }
     const T* VL = own ? Vs : Vx;
     const T* VR = own ? Vx : Vs;
-    T Fl[5];
-    if constexpr (kRef) {
-      T UL[5], UR[5];
-      prim_to_cons<T, kRef>(VL, UL);
-      prim_to_cons<T, kRef>(VR, UR);
-      rusanov_ref<T>(UL, UR, nh, area, Fl);
-    } else {
-      rusanov_fast<T>(VL, VR, nh, area, Fl);
-    }
+    T Fl[5], UL[5], UR[5];
+    prim_to_cons<T, true>(VL, UL);
+    prim_to_cons<T, true>(VR, UR);
+    rusanov_ref<T>(UL, UR, nh, area, Fl);
 #pragma unroll
     for (int k = 0; k < 5; k++) contrib[k] = own ? -double(Fl[k]) : double(Fl[k]);
   }
   // flux balance, accumulated in face-slot order: ((0 + c0) + c1) + ...
   double R[5];
 #pragma unroll
-  for (int k = 0; k < 5; k++) {
-    if constexpr (kRef) R[k] = quad_sum_ordered(contrib[k]);
-    else R[k] = quad_sum_tree(contrib[k]);
-  }
+  for (int k = 0; k < 5; k++) R[k] = quad_sum_ordered(contrib[k]);
 
   // ---- stage update (FP64); every lane computes it, lanes store by component ----
   const double vol = m.vol[c];
@@ -467,7 +415,7 @@ __global__ void __launch_bounds__(256) flux_update_kernel(MeshView<T> m, StageAr
     for (int k = 0; k < 5; k++) Unew[k] = U[k];
   }
   double Vn[5];
-  cons_to_prim<double, kRef>(Unew, Vn);
+  cons_to_prim<double, true>(Unew, Vn);
   if (!valid) return;
 #pragma unroll
   for (int k = 0; k < 5; k++) {

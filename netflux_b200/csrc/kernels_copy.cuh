@@ -101,7 +101,7 @@ __device__ __forceinline__ void gradient_copy_cell(const MeshView<float>& m, con
   const T ssum[3] = {(S[0][0] + S[1][0]) + (S[2][0] + S[3][0]), (S[0][1] + S[1][1]) + (S[2][1] + S[3][1]),
                      (S[0][2] + S[1][2]) + (S[2][2] + S[3][2])};
   const T hv = T(0.5) * nr_rcp(T(m.vol[c]));
-  const bool rat = a.barth && ratchet_on(a, c);
+  const bool rat = ratchet_on(a, c);
   auto variable = [&](int k, T vc, const T vo[4]) {
     T acc[3];
 #pragma unroll
@@ -116,21 +116,18 @@ __device__ __forceinline__ void gradient_copy_cell(const MeshView<float>& m, con
     T gr[4];
 #pragma unroll
     for (int q = 0; q < 4; q++) gr[q] = fma(g[2], d[q][2], fma(g[1], d[q][1], g[0] * d[q][0]));
-    T phi = T(1);
-    if (a.barth) {
-      T An = T(1), Dn = T(1);  // best ratio so far, starting at 1
+    T An = T(1), Dn = T(1);  // best ratio so far, starting at 1
 #pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const T d2 = gr[q];
-        const T A = d2 > T(0) ? vmax - vc : vc - vmin;
-        const T D = fabs(d2) + Gas<T>::eps;
-        const bool better = (d2 != T(0)) && (A * Dn < An * D);
-        An = better ? A : An;
-        Dn = better ? D : Dn;
-      }
-      phi = An * nr_rcp(Dn);
-      if (rat) phi = ratchet(a, size_t(k) * st + c, phi);
+    for (int q = 0; q < 4; q++) {
+      const T d2 = gr[q];
+      const T A = d2 > T(0) ? vmax - vc : vc - vmin;
+      const T D = fabs(d2) + Gas<T>::eps;
+      const bool better = (d2 != T(0)) && (A * Dn < An * D);
+      An = better ? A : An;
+      Dn = better ? D : Dn;
     }
+    T phi = An * nr_rcp(Dn);
+    if (rat) phi = ratchet(a, size_t(k) * st + c, phi);
 #pragma unroll
     for (int q = 0; q < 4; q++) fsc[size_t(q * 5 + k) * st] = fma(phi, gr[q], vc);
     if (a.phi32) a.phi32[k * st + c] = phi;
