@@ -764,9 +764,9 @@ __global__ void __launch_bounds__(128, 1) umma_gemm_test_kernel(const __nv_bfloa
 // box than the farthest of its nearest distances so far. The bound is computed
 // with the operations of the distance itself on differences that are no larger,
 // and rounding is monotone, so no distance below a passed one is missed: the result
-// is the minimum over all points, bit for bit. Unordered points only pass over
-// less. 1.3M cells and 36,864 wall points, the whole call: 17 ms
-// over all pairs, 2.4 ms so (of which 1.4 ms are its copies).
+// is the minimum over all points, bit for bit. 1.3M cells and 36,864 wall points, the
+// whole call: 17 ms over all pairs, 2.3 ms so (of which 1.4 ms are its copies). Points
+// or wall points in no order pass over little, and a block then compares all pairs.
 constexpr int WD_C = 32;  // points a cluster, clusters a group
 struct WallBox {
   float4 lo, hi;
@@ -827,19 +827,21 @@ __global__ void __launch_bounds__(256) wall_distance_kernel(const float* __restr
   const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
   const bool in = i < n;
-  if (__ballot_sync(0xffffffffu, in) == 0) return;
   const float px = in ? pts[3 * i] : 0.f, py = in ? pts[3 * i + 1] : 0.f, pz = in ? pts[3 * i + 2] : 0.f;
   const float4 p = make_float4(px, py, pz, 0.f);
   const WallBox mine = warp_box(in ? WallBox{p, p} : empty_box());
   float best = in ? kWallFar : 0.f;  // a lane without a point asks for nothing
   float limit = kWallFar;            // the largest best of the warp
+  auto compare = [&](float x, float y, float z) {
+    const float dx = px - x, dy = py - y, dz = pz - z;
+    best = fminf(best, fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
+  };
   auto visit = [&](int64_t c) {
     const float4* w = wall + c * WD_C;
 #pragma unroll 8
     for (int j = 0; j < WD_C; j++) {
       const float4 q = w[j];
-      const float dx = px - q.x, dy = py - q.y, dz = pz - q.z;
-      best = fminf(best, fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
+      compare(q.x, q.y, q.z);
     }
     limit = best;
 #pragma unroll
@@ -858,21 +860,59 @@ __global__ void __launch_bounds__(256) wall_distance_kernel(const float* __restr
     }
     return at;
   };
-  // the cluster that looks nearest first, for a close limit
-  float d = kWallFar;
-  int64_t at = 0;
-  for (int64_t g = lane; g < n_groups; g += 32) {
-    const float e = box_distance2(mine, group[g]);
-    if (e < d) {
-      d = e;
-      at = g;
+  auto visit_nearest = [&](const WallBox& b) {  // the cluster that looks nearest to b
+    float d = kWallFar;
+    int64_t at = 0;
+    for (int64_t g = lane; g < n_groups; g += 32) {
+      const float e = box_distance2(b, group[g]);
+      if (e < d) {
+        d = e;
+        at = g;
+      }
     }
-  }
-  const int64_t g0 = nearest(d, at);
-  {
-    const int64_t c = g0 * WD_C + lane;
+    const int64_t g0 = nearest(d, at), c = g0 * WD_C + lane;
     const bool has = c < n_clusters;
-    visit(nearest(has ? box_distance2(mine, box[c]) : kWallFar, has ? c : g0 * WD_C));
+    visit(nearest(has ? box_distance2(b, box[c]) : kWallFar, has ? c : g0 * WD_C));
+  };
+  visit_nearest(mine);  // first, for a close limit
+  // Where more than a quarter of the clusters may still hold a nearer point, for most
+  // of the block (points or wall points in no order), a visit at a time is slower than
+  // comparing all pairs with the wall points staged in shared memory.
+  // The whole call, 1.3M lattice points over 36,864: the points, the wall points or both
+  // shuffled 16.0, 14.5 and 16.2 ms, by visits alone 27.0, 25.8 and 27.0. The line at half
+  // of the clusters costs points far from all of them 10 % (409,600 points).
+  int64_t live = 0;
+  for (int64_t g = lane; g < n_groups; g += 32) live += !(box_distance2(mine, group[g]) >= limit);
+  live = int64_t(__reduce_add_sync(0xffffffffu, unsigned(live)));
+  bool many = 2 * live > n_groups;
+  if (many) {
+    for (int k = 4; k < 32; k += 8) {  // the nearest to some of the points, for a closer one
+      const float4 q = make_float4(__shfl_sync(0xffffffffu, px, k), __shfl_sync(0xffffffffu, py, k),
+                                   __shfl_sync(0xffffffffu, pz, k), 0.f);
+      visit_nearest(WallBox{q, q});
+    }
+    live = 0;
+    for (int64_t c = lane; c < n_clusters; c += 32) live += !(box_distance2(mine, box[c]) >= limit);
+    live = int64_t(__reduce_add_sync(0xffffffffu, unsigned(live)));
+    many = 4 * live > n_clusters;
+  }
+  if (2 * __syncthreads_count(many) > int(blockDim.x)) {
+    __shared__ __align__(16) float tile[3 * WD_C * WD_C];
+    for (int64_t t0 = 0; t0 < n_clusters * WD_C; t0 += WD_C * WD_C) {
+      const int count = int(n_clusters * WD_C - t0 < WD_C * WD_C ? n_clusters * WD_C - t0 : WD_C * WD_C);
+      __syncthreads();
+      for (int j = threadIdx.x; j < count; j += blockDim.x) {
+        const float4 q = wall[t0 + j];
+        tile[3 * j] = q.x;
+        tile[3 * j + 1] = q.y;
+        tile[3 * j + 2] = q.z;
+      }
+      __syncthreads();
+#pragma unroll 4
+      for (int j = 0; j < count; j++) compare(tile[3 * j], tile[3 * j + 1], tile[3 * j + 2]);
+    }
+    if (in) out[i] = sqrtf(best);
+    return;
   }
   for (int64_t gb = 0; gb < n_groups; gb += 32) {
     const float eg = gb + lane < n_groups ? box_distance2(mine, group[gb + lane]) : kWallFar;
