@@ -9,24 +9,9 @@
 // kernel. At 3.1M tets 140 and 186 us a launch.
 #pragma once
 
-#include "kernels_tile.cuh"
+#include "kernels_cell.cuh"
 
 namespace nf {
-
-// Ask the memory system to bring a line into L2 without holding a register;
-// the later load of the same address then waits on an L2 hit, not on DRAM.
-__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
-
-// The own-cell rows the stage update reads (Uin, Un, the local dt).
-__device__ __forceinline__ void prefetch_update_rows(const StageArgs& a, int c, int st) {
-#pragma unroll
-  for (int k = 0; k < 5; k++) prefetch_l2(a.Uin + size_t(k) * st + c);
-  if (a.scheme != 0 && a.stage != 0) {
-#pragma unroll
-    for (int k = 0; k < 5; k++) prefetch_l2(a.Un + size_t(k) * st + c);
-  }
-  if (a.local_dt) prefetch_l2(a.dt_local + c);
-}
 
 // kPipe: 0 one variable's loads at a time; 1 the next variable's loads in
 // flight during this one's arithmetic; 2 all five variables' loads issued

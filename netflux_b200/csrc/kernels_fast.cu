@@ -69,12 +69,10 @@ static void with_stage_kernel(int form, int tile, int mode, Fn&& f) {
     using std::integral_constant;
     // 256 threads: the largest tile whose lists fit three times in an SM's shared
     // memory (at 3.1M tets FP64 369 us a launch, 379 us at 192, 413 us at 160,
-    // 520 us or more at 128). Meshes whose tiles touch more than its rows hold
-    // (thin or badly ordered ones) take 128 with longer rows, then 64, whose rows
-    // hold whatever its cells can touch (17 values a cell).
+    // 520 us or more at 128). Small meshes whose tiles touch more than its rows hold
+    // (thin or flat ones) take 128 with longer rows.
     if (tile == 256) order(frm, integral_constant<int, 256>(), integral_constant<int, 6 * 256>());
-    else if (tile == 128) order(frm, integral_constant<int, 128>(), integral_constant<int, 8 * 128>());
-    else order(frm, integral_constant<int, 64>(), integral_constant<int, 17 * 64>());
+    else order(frm, integral_constant<int, 128>(), integral_constant<int, 8 * 128>());
   };
   if (form == kFormFp64) size(std::integral_constant<int, kFormFp64>());
   else if (form == kFormDelta) size(std::integral_constant<int, kFormDelta>());
@@ -101,6 +99,50 @@ cudaError_t stage_setup(int form, int tile, int mode, int max_smem, size_t smem,
 void launch_stage(int form, int tile, int mode, const MeshView<double>& m, const TileView& tv, const StageArgs& a,
                   size_t smem, cudaStream_t st) {
   with_stage_kernel(form, tile, mode, [&](auto k, auto, auto) { launch_pdl(k, tv.n_tiles, tile, smem, st, m, tv, a); });
+}
+// ---- the same stage by one thread a cell ----
+// f(form) or f(form, second order) with compile-time values
+template <typename Fn>
+static void with_form(int form, Fn&& f) {
+  using std::integral_constant;
+  if (form == kFormFp64) f(integral_constant<int, kFormFp64>());
+  else if (form == kFormDelta) f(integral_constant<int, kFormDelta>());
+  else f(integral_constant<int, kFormCopy>());
+}
+template <typename Fn>
+static void with_form_order(int form, bool second, Fn&& f) {
+  with_form(form, [&](auto frm) {
+    if (second) f(frm, std::true_type());
+    else f(frm, std::false_type());
+  });
+}
+void launch_cell_states(int form, const MeshView<double>& m, const StageArgs& a, cudaStream_t st) {
+  with_form(form, [&](auto f) {
+    launch_pdl(face_state_kernel<decltype(f)::value>, grid_for(m.n, 64), 64, 0, st, m, a);
+  });
+}
+void launch_cell_boundary(int form, bool second, const MeshView<double>& m, const TileView& tv, const StageArgs& a,
+                          cudaStream_t st) {
+  if (m.nb == 0) return;
+  with_form_order(form, second, [&](auto f, auto sec) {
+    launch_pdl(boundary_face_kernel<decltype(f)::value, decltype(sec)::value>, grid_for(m.nb, 128), 128, 0, st, m, tv, a);
+  });
+}
+// Blocks of 128 an SM should hold, which caps a thread's registers. Per launch at 1.3M
+// tets: FP64 second order 110 us at 6, 116 at 7, 125 at 8, 123 without a cap (first
+// order 91, 89, 95, 113); differences 121, 122, 111, 131 (first order 92, 87, 89, 103);
+// FP32 copies 92, 88, 85, 92.
+template <int kForm, bool kSecond>
+constexpr int kCellBlocks = kForm != kFormFp64 ? 8 : kSecond ? 6 : 7;
+void launch_cell_fluxes(int form, bool second, const MeshView<double>& m, const MeshView<float>& m32,
+                        const StageArgs& a, cudaStream_t st) {
+  with_form_order(form, second, [&](auto f, auto sec) {
+    constexpr int kF = decltype(f)::value;
+    constexpr bool kS = decltype(sec)::value;
+    auto* k = cell_flux_kernel<kF, kS, kCellBlocks<kF, kS>>;
+    if constexpr (kF == kFormFp64) launch_pdl(k, grid_for(m.n, 128), 128, 0, st, m, a);
+    else launch_pdl(k, grid_for(m.n, 128), 128, 0, st, m32, a);
+  });
 }
 // The form with FP32 copies under the Barth limiter: launch variants the tuner
 // times. 0 plain, 1 software-pipelined, 2 and 3 the same with registers capped

@@ -31,6 +31,13 @@ size_t stage_smem(int form, const Tiles& t, bool second);  // shared memory of a
 cudaError_t stage_setup(int form, int tile, int mode, int max_smem, size_t smem, int* blocks);
 void launch_stage(int form, int tile, int mode, const MeshView<double>& m, const TileView& tv, const StageArgs& a,
                   size_t smem, cudaStream_t st);
+// the same stage by one thread a cell (kernels_cell.cuh): limiter and face states
+// (second order), then boundary fluxes, fluxes and update
+void launch_cell_states(int form, const MeshView<double>& m, const StageArgs& a, cudaStream_t st);
+void launch_cell_boundary(int form, bool second, const MeshView<double>& m, const TileView& tv, const StageArgs& a,
+                          cudaStream_t st);
+void launch_cell_fluxes(int form, bool second, const MeshView<double>& m, const MeshView<float>& m32,
+                        const StageArgs& a, cudaStream_t st);
 // the form with FP32 copies under the Barth limiter (kernels_copy.cuh)
 void launch_gradient_copy(const MeshView<float>& m, const StageArgs& a, Launch l, int variant);
 void launch_flux_copy(const MeshView<float>& m, const StageArgs& a, Launch l, int variant);

@@ -274,6 +274,7 @@ struct nf_solver {
   DevBuf<int> cut_cell, far_id, tile_node;
   DevBuf<double4> b_geo;
   DevBuf<int2> b_ref;
+  bool tiled = false;  // stages by the stage kernel, else by kernels of one thread a cell
   int tile = 0, n_tiles = 0, ahead = 0;
   int stage_mode = 0;  // kModeFirst ... kModeGeneral
   size_t stage_smem = 0;
@@ -389,7 +390,17 @@ struct nf_solver {
   // of 153,600 (1.4 waves) 100.3 -> 97.7, but of 393,216 (3.5 waves) 159 -> 163 and of
   // 3.1M (28 waves) 1.100 -> 1.132 ms.
   static constexpr int kGhostWaves = 2;
-  bool own_ghosts() const { return n_tiles <= kGhostWaves * ahead && !copy_barth(); }  // the stage kernel leaves them
+  // The stage kernel takes up to one wave of tiles whatever they cut (launches count
+  // most), and in second order any number of tiles of 256 cells that cut at most
+  // kMaxCut faces a cell. Else kernels of one thread a cell (kernels_cell.cuh). A step,
+  // stage kernel against those: FP64 48,000 tets (0.80 cut faces a cell) 42.1 / 50.6 us;
+  // 1.3M (0.88) 507 / 514, 3.1M (0.74) 1,104 / 1,134; 546,750 flat 2:1 (0.95) 247 / 241,
+  // 3:1 (1.00) 272 / 241; 1.3M flat 10:1 (1.62, in tiles of 128) 873 / 496, flat 50:1
+  // (2.95, of 64) 2,039 / 502. Differences at 1.3M: 0.88 483 / 470, 1.00 515 / 459, 1.62
+  // 698 / 452; FP32 copies 338 / 349, 357 / 342, 433 / 341. First order FP64: 93,750 tets
+  // (0.8 waves) 32.0 / 34.2, 162,000 (1.4) 50.2 / 44.9, 1.3M 325 / 257, 3.1M 719 / 573.
+  static constexpr double kMaxCut = 0.9;
+  bool own_ghosts() const { return tiled && n_tiles <= kGhostWaves * ahead; }  // the stage kernel leaves them
   bool ghosts_ready = false;
   double* vgbuf(int i) { return i && fast() ? vgb.p : vg.p; }
   float* vg32buf(int i) { return i ? vg32b.p : vg32.p; }
@@ -767,9 +778,9 @@ struct nf_solver {
           nf::launch_gradient_field(form(), view64(), view32(), a, stream);
           prof_end();
         }
+        a.fs32 = fs32.p;
+        a.fb32 = fb32.p;
         if (copy_barth()) {
-          a.fs32 = fs32.p;
-          a.fb32 = fb32.p;
           prof_begin(NF_KERNEL_GRADIENT);
           nf::launch_gradient_copy(view32(), a, nf::Launch{kgrad.block, stream}, kgrad.variant);
           prof_end();
@@ -778,6 +789,18 @@ struct nf_solver {
           prof_end();
           prof_begin(NF_KERNEL_FLUX);
           nf::launch_flux_copy(view32(), a, nf::Launch{kflux.block, stream}, kflux.variant);
+          prof_end();
+        } else if (!tiled) {
+          if (a.second_order) {
+            prof_begin(NF_KERNEL_GRADIENT);
+            nf::launch_cell_states(form(), view64(), a, stream);
+            prof_end();
+          }
+          prof_begin(NF_KERNEL_OTHER);
+          nf::launch_cell_boundary(form(), a.second_order != 0, view64(), tiles(), a, stream);
+          prof_end();
+          prof_begin(NF_KERNEL_FLUX);
+          nf::launch_cell_fluxes(form(), a.second_order != 0, view64(), view32(), a, stream);
           prof_end();
         } else {
           prof_begin(NF_KERNEL_FLUX);
@@ -1399,51 +1422,61 @@ nf_solver* nf_create(const nf_mesh* h, const nf_params* params) {
     }
 
     if (fast) {
-      if (s->copy_barth() || p.keep_stage_fields) {  // what the stage kernel does not read
-        s->gcode.upload(h_gcode, st);
-        s->cnode.upload(h_cnode, st);
-        s->nbvf.upload(h_nbvf, st);
-      }
       if (!s->copy_barth()) {
-        int max_smem = 0;
+        int max_smem = 0, n_sm = 0;
         ck(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device), "attr");
+        ck(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, s->device), "attr");
         const bool second = p.spatial_order == NF_SECOND_ORDER;
         nf::Tiles tl;
-        for (int tile : {256, 128, 64}) {
+        // tiles of 128 only where they can be a wave at most (no form holds more than 1024 threads an SM)
+        for (int tile : {256, 128}) {
+          if (s->stage_smem > 0 || (tile == 128 && s->n > 1024 * n_sm)) break;
           tl = nf::build_tiles(s->n, stride, tile, h_nbvf, h_nbsf, h_cnode, h_gcode, hb_cell);
           const size_t b = nf::stage_smem(s->form(), tl, second);
-          if (b > 0 && b <= size_t(max_smem)) break;
+          if (b <= size_t(max_smem)) s->stage_smem = b;
         }
         bool open = false;  // some face is not listed
+        int64_t cut = 0;    // faces between two tiles, from either side
         for (int ti = 0, cs = 0; ti < tl.n_tiles; ti++) {
           const int64_t c0 = int64_t(ti) * tl.tile, c1 = std::min(N, c0 + tl.tile);
           while (m.case_offsets[size_t(cs) + 1] <= c0) cs++;
           open = open || tl.head[size_t(ti)].open;
+          cut += tl.head[size_t(ti)].ncut;
           tl.head[size_t(ti)].case_id = m.case_offsets[size_t(cs) + 1] >= c1 ? cs : -1;
         }
         s->tile = tl.tile;
         s->n_tiles = tl.n_tiles;
-        s->stage_smem = nf::stage_smem(s->form(), tl, second);
-        int per_sm = 0, n_sm = 0;
-        ck(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, s->device), "attr");
+        int per_sm = 0;
         const bool ratchets = p.limiter == NF_LIMITER_BARTH && (p.limiter_ratchet_step > 0 || p.limiter_ratchet_drop > 0.0);
         auto setup = [&](int mode) {
           s->stage_mode = mode;
           ck(nf::stage_setup(s->form(), s->tile, mode, max_smem, s->stage_smem, &per_sm), "stage kernel set-up");
           s->ahead = std::max(1, per_sm) * n_sm;
         };
-        if (!second) setup(nf::kModeFirst);
-        else if (open || ratchets || p.keep_stage_fields) setup(nf::kModeGeneral);
-        else setup(nf::kModePlain);
-        if (s->stage_mode == nf::kModePlain && s->own_ghosts()) setup(nf::kModeGhosts);
-        s->tile_head.upload(tl.head, st);
-        s->tile_code.upload(tl.code, st);
-        s->tile_vert.upload(tl.vert, st);
-        s->cut_cell.upload(tl.cut_cell, st);
-        s->cut_nb.upload(tl.cut_nb, st);
-        s->far_id.upload(tl.far_id, st);
-        s->tile_node.upload(tl.node_id, st);
+        if (s->stage_smem > 0) {
+          if (!second) setup(nf::kModeFirst);
+          else if (open || ratchets || p.keep_stage_fields) setup(nf::kModeGeneral);
+          else setup(nf::kModePlain);
+          const bool one_wave = s->n_tiles <= s->ahead;
+          s->tiled = one_wave || (second && s->tile == 256 && double(cut) <= nf_solver::kMaxCut * double(N));
+        }
+        if (s->tiled && s->stage_mode == nf::kModePlain && s->own_ghosts()) setup(nf::kModeGhosts);
+        if (s->tiled) {
+          s->tile_head.upload(tl.head, st);
+          s->tile_code.upload(tl.code, st);
+          s->tile_vert.upload(tl.vert, st);
+          s->cut_cell.upload(tl.cut_cell, st);
+          s->cut_nb.upload(tl.cut_nb, st);
+          s->far_id.upload(tl.far_id, st);
+          s->tile_node.upload(tl.node_id, st);
+        }
       }
+      if (!s->tiled || p.keep_stage_fields) {  // what the stage kernel does not read
+        s->gcode.upload(h_gcode, st);
+        s->cnode.upload(h_cnode, st);
+        s->nbvf.upload(h_nbvf, st);
+      }
+      if (!s->tiled) s->nbsf.upload(h_nbsf, st);
       std::vector<double4> h_bgeo(static_cast<size_t>(nbf));
       std::vector<int2> h_bref(static_cast<size_t>(nbf));
       for (int b = 0; b < nbf; b++) {
@@ -1468,12 +1501,15 @@ nf_solver* nf_create(const nf_mesh* h, const nf_params* params) {
     s->dS.upload(h_dS, st);
     s->patches.upload(h_pb, st);
     const bool fp32_fields = p.precision == NF_PREC_MIXED || p.precision == NF_PREC_MIXED32;
-    if (s->copy_barth()) {
-      s->fs32.alloc(size_t(20) * stride);
-      s->fs32.zero(st);
+    // face states and boundary fluxes of the kernels that exchange them through HBM
+    const bool fs_hbm = !s->tiled && (!fast || p.spatial_order == NF_SECOND_ORDER);
+    if (fp32_fields && !s->tiled) {
+      if (fs_hbm) {
+        s->fs32.alloc(size_t(20) * stride);
+        s->fs32.zero(st);
+      }
       s->fb32.alloc(size_t(5) * s->bstride);
       s->fb32.zero(st);
-      s->nbsf.upload(h_nbsf, st);
     }
     if (p.precision == NF_PREC_MIXED32) {
       s->V32a.alloc(size_t(5) * stride);
@@ -1501,9 +1537,11 @@ nf_solver* nf_create(const nf_mesh* h, const nf_params* params) {
       s->vgb.alloc(size_t(5) * s->bstride);
       s->vgb.zero(st);
     }
-    if (!fast) {
-      s->fs.alloc(size_t(20) * stride);
-      s->fs.zero(st);
+    if (!fp32_fields && !s->tiled) {
+      if (fs_hbm) {
+        s->fs.alloc(size_t(20) * stride);
+        s->fs.zero(st);
+      }
       s->fb.alloc(size_t(5) * s->bstride);
       s->fb.zero(st);
     }

@@ -1,6 +1,6 @@
 """The NF_DEBUG build on what the golden cases of test_debug_build.py do not reach: the form with FP32
-copies with and without the limiter, first order, unlisted faces, kept stage fields, and meshes whose
-tiles have 128 and 64 cells. Valid meshes: nothing reported, the release build's bits."""
+copies with and without the limiter, first order, unlisted faces, kept stage fields, a mesh whose tiles
+have 128 cells, and one that runs by kernels of one thread a cell. Valid meshes: nothing reported, the release build's bits."""
 import os
 import subprocess
 import sys
