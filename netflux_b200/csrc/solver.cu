@@ -386,20 +386,25 @@ struct nf_solver {
   // primitives are in place, and whatever else writes primitives clears it.
   // Up to kGhostWaves waves of tiles a kernel of its own (4 us a stage, mostly
   // launch) costs more than the boundary tiles' longer stay, beyond it less:
-  // separate against left by the stage kernel, a step of 48,000 tets 45.8 -> 41.6 us,
-  // of 153,600 (1.4 waves) 100.3 -> 97.7, but of 393,216 (3.5 waves) 159 -> 163 and of
-  // 3.1M (28 waves) 1.100 -> 1.132 ms.
+  // separate against left by the stage kernel, a step of FP64 48,000 tets 46.5 / 42.3
+  // us, 96,000 (0.8 waves) 57.0 / 52.6, 165,888 (1.5) 85.0 / 84.8, 324,000 (2.9) 142.0 /
+  // 144.3, 546,750 (4.8) 240.7 / 252.1; differences 44.7 / 41.7, 54.5 / 50.8, 81.1 / 82.5,
+  // 131.9 / 134.7, 230.4 / 242.1; FP32 copies without the limiter 37.9 / 33.8, 47.1 /
+  // 43.3, 61.1 / 56.8 (1.1 waves), 96.6 / 93.5 (2.1), 164.9 / 172.7 (3.6).
   static constexpr int kGhostWaves = 2;
   // The stage kernel takes up to one wave of tiles whatever they cut (launches count
   // most), and in second order any number of tiles of 256 cells that cut at most
-  // kMaxCut faces a cell. Else kernels of one thread a cell (kernels_cell.cuh). A step,
-  // stage kernel against those: FP64 48,000 tets (0.80 cut faces a cell) 42.1 / 50.6 us;
-  // 1.3M (0.88) 507 / 514, 3.1M (0.74) 1,104 / 1,134; 546,750 flat 2:1 (0.95) 247 / 241,
-  // 3:1 (1.00) 272 / 241; 1.3M flat 10:1 (1.62, in tiles of 128) 873 / 496, flat 50:1
-  // (2.95, of 64) 2,039 / 502. Differences at 1.3M: 0.88 483 / 470, 1.00 515 / 459, 1.62
-  // 698 / 452; FP32 copies 338 / 349, 357 / 342, 433 / 341. First order FP64: 93,750 tets
-  // (0.8 waves) 32.0 / 34.2, 162,000 (1.4) 50.2 / 44.9, 1.3M 325 / 257, 3.1M 719 / 573.
-  static constexpr double kMaxCut = 0.9;
+  // kMaxCut faces a cell (kMaxCutFew up to kGhostWaves waves, where a launch still
+  // counts). Else kernels of one thread a cell (kernels_cell.cuh). A step, stage kernel
+  // against those: FP64 48,000 tets (0.80 cut faces a cell) 42.1 / 50.6 us; 236,196
+  // (0.98) 112.9 / 118.2; 559,872 (0.94) 237.5 / 242.0, 546,750 flat 3:1 (1.00) 272 /
+  // 241, 1.3M (0.88) 507 / 514, flat 3:1 (1.01) 580 / 499, flat 10:1 (1.62, in tiles of
+  // 128) 873 / 496, flat 50:1 (2.95, of 64) 2,039 / 502; 3.1M (0.74) 1,104 / 1,134.
+  // Differences 127,776 (1.03) 70.8 / 74.6, 215,622 (1.12) 101.8 / 105.0, 1.3M 483 / 470,
+  // 515 / 459, 698 / 452; FP32 copies 1.3M 338 / 349, 357 / 342, 433 / 341. First order
+  // FP64: 93,750 tets (0.8 waves) 32.0 / 34.2, 162,000 (1.4) 50.2 / 44.9, 1.3M 325 / 257,
+  // 3.1M 719 / 573.
+  static constexpr double kMaxCut = 1.0, kMaxCutFew = 1.15;
   bool own_ghosts() const { return tiled && n_tiles <= kGhostWaves * ahead; }  // the stage kernel leaves them
   bool ghosts_ready = false;
   double* vgbuf(int i) { return i && fast() ? vgb.p : vg.p; }
@@ -1458,7 +1463,8 @@ nf_solver* nf_create(const nf_mesh* h, const nf_params* params) {
           else if (open || ratchets || p.keep_stage_fields) setup(nf::kModeGeneral);
           else setup(nf::kModePlain);
           const bool one_wave = s->n_tiles <= s->ahead;
-          s->tiled = one_wave || (second && s->tile == 256 && double(cut) <= nf_solver::kMaxCut * double(N));
+          const double most = s->n_tiles <= nf_solver::kGhostWaves * s->ahead ? nf_solver::kMaxCutFew : nf_solver::kMaxCut;
+          s->tiled = one_wave || (second && s->tile == 256 && double(cut) <= most * double(N));
         }
         if (s->tiled && s->stage_mode == nf::kModePlain && s->own_ghosts()) setup(nf::kModeGhosts);
         if (s->tiled) {

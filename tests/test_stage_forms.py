@@ -29,8 +29,8 @@ def _companion(kind):
         m = mg.box_tet_mesh(60, 6, 6, hi=(1.0, 0.02, 1.0))
     elif kind == "order":  # cells in random order: no tile holds what its cells touch, a thread a cell
         m = _shuffled(7, 24)
-    elif kind == "flat":  # 162,000 tets flattened 6:1: more than a wave of tiles, cut too often for them
-        m = mg.box_tet_mesh(30, 30, 30, hi=(1.0, 1.0 / 6.0, 1.0))
+    elif kind == "flat":  # 162,000 tets flattened 10:1: more than a wave of tiles, cut too often for them
+        m = mg.box_tet_mesh(30, 30, 30, hi=(1.0, 0.1, 1.0))
     else:  # 384,000 tets more: past the size up to which the stage kernel leaves the ghosts
         m = mg.cube_mesh(40)
     return S.Mesh.from_tet_mesh(m), _state(m)
