@@ -66,7 +66,7 @@ def parse():
     ap.add_argument("--variant", type=int, default=0, help="with --block: fast-kernel variant")
     ap.add_argument("--shapes", type=int, nargs=4, default=None, metavar=("GB", "GV", "FB", "FV"),
                     help="fix the gradient and flux kernels' (block, variant) separately (no tuning); "
-                         "they run where the fused stage kernel does not: --precision mixed32")
+                         "they run with --precision mixed32")
     return ap.parse_args()
 
 
@@ -186,8 +186,8 @@ def algorithmic_bytes(n_cells: int, n_faces: int, n_boundary: int, n_nodes: int,
                       local_dt: bool):
     """Compulsory HBM bytes of one launch of each kernel where limiter and flux are kernels of their
     own, which exchange four face states a cell (every datum read or written once, averaged over the
-    three stages). FP32 copies under the Barth limiter run that way; the FP64 and difference forms'
-    figures say what the fused kernel (stage_bytes) saves.
+    three stages): FP32 copies under the Barth limiter, and meshes that the fused kernel does not take
+    (their limiter kernel needs neither vertices nor code nor volume: 28 B a cell less than said here).
 
     FP64, per cell:
       gradient: V (40), 4 vertex ids (16), 4 neighbour ids (16), face code (4), vol (8), writes 4
@@ -230,8 +230,8 @@ STAGE_DRAM_BYTES_PER_CELL = {"fp64": 836.7e6 / 3145728, "mixed": 805.1e6 / 31457
 # them (FP32 copies, shapes 64 9 128 9; stages 426.4 / 427.1 / 426.2 and 751.2 / 957.5 / 856.5 MB).
 MEASURED_DRAM_BYTES_PER_CELL = {("mixed32", "gradient"): 426.6e6 / 3145728,
                                 ("mixed32", "flux"): 855.0e6 / 3145728}
-# Forms whose kernels come in several launch shapes (nf_tune times them); the others' stage kernel
-# has the one that its mesh calls for, and their lines carry no shapes.
+# Forms whose kernels come in several launch shapes (nf_tune times them); the others' kernels have
+# the one that the mesh calls for, and their lines carry no shapes.
 FORMS_WITH_SHAPES = ("mixed32",)
 
 

@@ -335,7 +335,7 @@ int nf_synchronize(nf_solver* s);
  * pipelined, 6 and 7 all before any arithmetic, 8 and 9 after L2 prefetches of
  * the cell's own rows) and a register cap for occupancy (none, variants 0-1 and
  * 6; 8 resident 128-thread blocks, variants 2-3 and 8; 9, variants 4-5 and 9; 5,
- * variant 7). The other forms' stage kernel has one shape, which follows from the
+ * variant 7). The other forms' kernels have one shape, which follows from the
  * mesh, so for them nothing is timed. config (may be NULL) receives {gradient
  * block, gradient variant, flux block, flux variant}. The state is unchanged. The
  * reference has no counterpart (it runs on one CPU thread). */

@@ -4,9 +4,10 @@
 // the limiter's switches (a hundred steps turn 2e-8 into some 1e-6 of the state's
 // norm, and a thousand times that in single cells), so another arrangement of the
 // same reconstruction, such as the stage kernel's, gives results that differ from
-// these by as much as either is in error. The other forms, and this one without
-// the limiter or in first order, have no such amplification and take the stage
-// kernel. At 3.1M tets 140 and 186 us a launch.
+// these by up to 1e-3 in a cell after a hundred steps. Which of the two is nearer to
+// FP64 has not been measured; until it is, the form keeps its operations. The other
+// forms, and this one without the limiter or in first order, have no such
+// amplification. At 3.1M tets 140 and 186 us a launch.
 #pragma once
 
 #include "kernels_cell.cuh"

@@ -17,11 +17,13 @@
 // stage is one launch (two where the ghosts have their own kernel). Separate
 // limiter and flux kernels wrote and re-read 20 face states a cell (160 B out and
 // 160 B in, FP64) in four launches. The price is the limiter of the cut faces'
-// outside cells, 0.9 a cell at 256 cells a tile.
+// outside cells, 0.7 to 0.9 a cell at 256 cells a tile on meshes of compact cells (0.70
+// at 393,216 tets of the channel, 0.74 at 3.1M, 0.80 in the cube of 48,000), more where
+// cells are flat or stretched: those meshes go by one thread a cell (kernels_cell.cuh;
+// solver.cu has the rule).
 //
-// A step, against those kernels: FP64 48,000 tets 62 -> 42 us, 153,600 tets (thin
-// tube) 95 -> 98 us, 3.1M tets 1.218 -> 1.100 ms; FP32 copies without the limiter,
-// 3.1M, 0.80 -> 0.76 ms; difference form 96,000 tets 74 -> 49 us, 393,216 183 -> 159
+// A step, against those kernels: FP64 48,000 tets 62 -> 42 us, 3.1M tets 1.218 ->
+// 1.100 ms; FP32 copies without the limiter, 3.1M, 0.80 -> 0.73 ms; difference form 96,000 tets 74 -> 49 us, 393,216 183 -> 159
 // us, 3.1M 1.051 -> 1.050 ms. Bound by latency: about 1,860 instructions a cell at 24
 // warps an SM (80 registers, three blocks), 43 % of issue slots and 33 % of the
 // FP64 pipe busy; of 12.5 cycles between a warp's instructions 3 wait for global
